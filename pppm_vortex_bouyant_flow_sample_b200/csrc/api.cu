@@ -206,6 +206,8 @@ cudaError_t alloc_grid_side(pppm_scene *s) {
         pool += 2 * 3 * (size_t)s->lv[l].cells;
         d = (d / 2 == 0) ? 1 : d / 2;
     }
+    PPPM_CUDA_TRY(pppm::mg_tail_prepare());
+    PPPM_CUDA_TRY(pppm::mg_sweep_prepare());
     PPPM_CUDA_TRY(dalloc(&s->mg_pool, pool));
     float *p = s->mg_pool;
     for (int l = 0; l < s->levels; l++) {
@@ -242,18 +244,11 @@ cudaError_t alloc_grid_side(pppm_scene *s) {
     PPPM_CUDA_TRY(dalloc(&s->dparams, 1));
     PPPM_CUDA_TRY(dalloc(&s->norms, 2));
     PPPM_CUDA_TRY(dalloc(&s->pair_count, 1));
-    if (s->levels >= 2) {
-        const int dc = (int)s->lv[s->levels - 1].d;
-        const size_t cc = (size_t)dc * dc * dc;
-        PPPM_CUDA_TRY(dalloc(&s->coarse_op, cc * cc));
-    }
     // initialise on a private stream (no device-wide synchronisation)
     cudaStream_t st = nullptr;
     PPPM_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     cudaError_t e = cudaMemsetAsync(s->mflag, 0, sizeof(uint32_t) * s->C, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->dparams, 0, sizeof(pppm::DevParams), st);
-    if (e == cudaSuccess && s->coarse_op)
-        e = pppm::build_coarse_operator((int)s->lv[s->levels - 1].d, s->coarse_op, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     cudaStreamDestroy(st);
     return e;
@@ -283,7 +278,6 @@ void destroy_scene(pppm_scene *s) {
     cudaFree(s->dparams);
     cudaFree(s->norms);
     cudaFree(s->pair_count);
-    cudaFree(s->coarse_op);
     if (s->mg_graph) cudaGraphExecDestroy(s->mg_graph);
     pppm::free_buoyancy(s->buoy);
     delete s;
@@ -868,7 +862,7 @@ struct pppm_mg {
     float *x2_pool = nullptr;               // second x copies of the blocked-smoother levels
     uint32_t *err = nullptr;                // its device error flag
     double *r64 = nullptr, *e64 = nullptr;  // residual of the initial guess, its correction
-    double *coarse_op = nullptr;            // coarsest-level operator (levels >= 2)
+    float *scratch = nullptr;               // second copy of x while a level is smoothed
     cudaGraphExec_t graph = nullptr;        // reference-schedule solve of r64 into e64, captured on first use
     unsigned graph_kernels = 0;
     uint32_t n = 0;
@@ -927,21 +921,17 @@ extern "C" pppm_status pppm_mg_create(uint32_t n, void *stream, pppm_mg **out) {
     if (e == cudaSuccess) e = dalloc(&P.norms, 2);
     if (e == cudaSuccess) e = dalloc(&m->r64, P.lv[0].cells);
     if (e == cudaSuccess) e = dalloc(&m->e64, P.lv[0].cells);
-    if (e == cudaSuccess && P.levels >= 2) {
-        // the coarsest solve from x = 0 as one precomputed linear map, as for scenes
-        const uint32_t cc = P.lv[P.levels - 1].cells;
-        e = dalloc(&m->coarse_op, (size_t)cc * cc);
-        if (e == cudaSuccess) e = pppm::build_coarse_operator((int)P.lv[P.levels - 1].d, m->coarse_op, P.st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(P.st);
-        P.coarse_op = m->coarse_op;
-    }
+    if (e == cudaSuccess) e = dalloc(&m->scratch, P.lv[0].cells);
+    P.scratch = m->scratch;
+    if (e == cudaSuccess) e = pppm::mg_tail_prepare();
+    if (e == cudaSuccess) e = pppm::mg_sweep_prepare();
     if (e != cudaSuccess) {
         pppm_status st = cuda_fail("pppm_mg_create", e);
         cudaFree(m->pool);
         cudaFree(P.norms);
         cudaFree(m->r64);
         cudaFree(m->e64);
-        cudaFree(m->coarse_op);
+        cudaFree(m->scratch);
         delete m;
         return st;
     }
@@ -966,8 +956,8 @@ extern "C" pppm_status pppm_mg_create(uint32_t n, void *stream, pppm_mg **out) {
             cudaFree(P.norms);
             cudaFree(m->r64);
             cudaFree(m->e64);
-            cudaFree(m->coarse_op);
-            cudaFree(m->x2_pool);
+            cudaFree(m->scratch);
+                cudaFree(m->x2_pool);
             cudaFree(m->err);
             delete m;
             return st;
@@ -986,7 +976,7 @@ extern "C" pppm_status pppm_mg_destroy(pppm_mg *m) {
     cudaFree(m->plan.norms);
     cudaFree(m->r64);
     cudaFree(m->e64);
-    cudaFree(m->coarse_op);
+    cudaFree(m->scratch);
     cudaFree(m->x2_pool);
     cudaFree(m->err);
     delete m;
@@ -1063,7 +1053,6 @@ extern "C" pppm_status pppm_mg_vcycle(pppm_mg *m, double *x, const double *b, in
         P.tb_maps[l] = m->plan.tb_maps[level + l];
         P.tb_zchunk[l] = m->plan.tb_zchunk[level + l];
     }
-    P.coarse_op = (P.levels >= 2) ? m->coarse_op : nullptr;
     const size_t C = P.lv[0].cells;
     ::pppm::note_launch();
     residual64_kernel<<<(unsigned)((C + 255) / 256), 256, 0, P.st>>>(x, b, m->r64, P.lv[0].b, (int)P.lv[0].d);

@@ -10,7 +10,8 @@
 // b - (sum_nbr - 6x); restriction 0.5 * sum of the 8 children; prolongation
 // by injection; 100 Jacobi sweeps on the coarsest level
 // (MG/MultiGrid_kernel.cu:422-498; the reference updates in place from 512
-// racing threads, Jacobi is its race-free reading).
+// racing threads, Jacobi is its race-free reading).  The levels of edge <= 32
+// run in one launch (mg_tail.cu); the kernels here take the larger ones.
 //
 // Precision: the full-multigrid part runs in FP32.  The final V-cycle runs as
 // an FP64 defect correction — r = b - A psi in FP64, an FP32 V-cycle on
@@ -19,11 +20,9 @@
 // iteration.  The coarsest solve is FP64.  Every kernel handles the three
 // potential components of a scene in one launch (grid y = component).
 //
-// Where the level's edge allows, the half sweeps and the prolongation take a
-// group of 4 consecutive cells of a row per thread and the restriction a pair
-// of coarse cells, with 128-bit loads; their values equal the one-cell
-// kernels' bit for bit.  The temporally blocked smoother of mg_tb.cu is
-// opt-in (PPPM_MG_TB), as it measured slower inside a whole solve.
+// Levels of edge > 32 run one kernel per red-black sweep (mg_sweep.cu); the
+// restriction takes a pair of coarse cells per thread with 128-bit loads.  The
+// temporally blocked smoother of mg_tb.cu is opt-in (PPPM_MG_TB).
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -37,8 +36,6 @@ namespace pppm {
 
 namespace {
 
-constexpr float kOmegaF = 1.43f;
-constexpr float kOneMinusOmegaF = 1.0f - 1.43f;  // formed in float, MG/MultiGrid_kernel.cu:766
 constexpr int kMGThreads = 256;
 
 __device__ __forceinline__ float nb_sum(const float *__restrict__ x, int i, int j, int k, int d, size_t c) {
@@ -86,106 +83,15 @@ __device__ __forceinline__ void split3(uint32_t t, int a, int d, int la, int ld,
     }
 }
 
-// The SOR update of one cell from its neighbour sum and right-hand side
-// (MG/MultiGrid_kernel.cu:766, omega = 1.43f), one expression for every
-// smoother kernel so that they round alike.
-__device__ __forceinline__ float sor_update(float x, float nb, float b) {
-    const float r = nb - b;
-    return kOneMinusOmegaF * x + (kOmegaF * r) * (1.0f / 6.0f);
-}
-
-// One half sweep over the cells with (i+j+k) % 2 == color.
-__global__ void __launch_bounds__(kMGThreads)
-rbsor_kernel(float *__restrict__ x, const float *__restrict__ b, int d, int color, int ld) {
-    const int half = d >> 1;
-    const uint32_t per = (uint32_t)half * d * d;
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= per) return;
-    const size_t comp = blockIdx.y;
-    const size_t cells = (size_t)d * d * d;
-    float *xc = x + comp * cells;
-    const float *bc = b + comp * cells;
-    int ih, j, k;
-    split3(t, half, d, ld > 0 ? ld - 1 : -1, ld, ih, j, k);
-    const int i = 2 * ih + ((j + k + color) & 1);
-    const size_t c = ((size_t)k * d + j) * d + i;
-    xc[c] = sor_update(xc[c], nb_sum(xc, i, j, k, d, c), bc[c]);
-}
-
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 
-// The same half sweep with a thread per group of 4 consecutive cells of a
-// row (edge a multiple of 4): it updates the group's 2 cells of the colour
-// from 128-bit loads of its row, the rows and planes either side and b, plus
-// one scalar either side, with nb_sum's terms in nb_sum's order (the values
-// equal rbsor_kernel's bit for bit).  Half the threads of rbsor_kernel, and
-// every loaded sector fully used.
-__global__ void __launch_bounds__(kMGThreads)
-rbsor4_kernel(float *__restrict__ x, const float *__restrict__ b, int d, int color, int ld) {
-    const int q = d >> 2;  // groups per row
-    const uint32_t per = (uint32_t)q * d * d;
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= per) return;
-    const size_t comp = blockIdx.y;
-    const size_t cells = (size_t)d * d * d, dd = (size_t)d * d;
-    float *xc = x + comp * cells;
-    const float *bc = b + comp * cells;
-    int g, j, k;
-    split3(t, q, d, ld >= 2 ? ld - 2 : -1, ld, g, j, k);
-    const int i0 = 4 * g;
-    const size_t c = ((size_t)k * d + j) * d + i0;
-    const bool odd = ((j + k + color) & 1) != 0;  // the colour's cells: i0 + odd, i0 + odd + 2
-    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 v = ld4(xc + c);
-    const float xl = i0 > 0 ? xc[c - 1] : 0.f;
-    const float xr = i0 + 4 < d ? xc[c + 4] : 0.f;
-    const float4 up = (j < d - 1) ? ld4(xc + c + d) : z4;
-    const float4 dn = (j > 0) ? ld4(xc + c - d) : z4;
-    const float4 fr = (k > 0) ? ld4(xc + c - dd) : z4;
-    const float4 bk = (k < d - 1) ? ld4(xc + c + dd) : z4;
-    const float4 bb = ld4(bc + c);
-    const float nb_lo = (((odd ? v.x : xl) + (odd ? v.z : v.y)) + ((odd ? up.y : up.x) + (odd ? dn.y : dn.x))) +
-                        ((odd ? fr.y : fr.x) + (odd ? bk.y : bk.x));
-    const float nb_hi = (((odd ? v.z : v.y) + (odd ? xr : v.w)) + ((odd ? up.w : up.z) + (odd ? dn.w : dn.z))) +
-                        ((odd ? fr.w : fr.z) + (odd ? bk.w : bk.z));
-    const int o = odd ? 1 : 0;
-    xc[c + o] = sor_update(odd ? v.y : v.x, nb_lo, odd ? bb.y : bb.x);
-    xc[c + o + 2] = sor_update(odd ? v.w : v.z, nb_hi, odd ? bb.w : bb.z);
-}
-
 // Residual at the fine level restricted to the coarse level in one pass:
-// bc = 0.5 * sum over the 8 children of (bf - (sum_nbr(xf) - 6 xf)).
-__global__ void __launch_bounds__(kMGThreads)
-resid_restrict_kernel(const float *__restrict__ xf, const float *__restrict__ bf, float *__restrict__ bc,
-                      int dc, int x_zero, int ldc) {
-    const uint32_t per = (uint32_t)dc * dc * dc;
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= per) return;
-    const size_t comp = blockIdx.y;
-    const int df = 2 * dc;
-    const size_t fcells = (size_t)df * df * df;
-    const float *x = xf + comp * fcells;
-    const float *b = bf + comp * fcells;
-    int ic, jc, kc;
-    split3(t, dc, dc, ldc, ldc, ic, jc, kc);
-    float sum = 0.f;
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-        const int i = 2 * ic + (q & 1), j = 2 * jc + ((q >> 1) & 1), k = 2 * kc + (q >> 2);
-        const size_t c = ((size_t)k * df + j) * df + i;
-        float r = b[c];
-        if (!x_zero) r -= nb_sum(x, i, j, k, df, c) - 6.f * x[c];
-        sum += r;
-    }
-    bc[comp * per + t] = sum * 0.5f;
-}
-
-// The same with a thread per pair of coarse cells along x (coarse edge even):
-// their 16 fine children, 4 consecutive cells in each of the 4 fine rows
-// (j, k) in {2jc, 2jc+1} x {2kc, 2kc+1}, read with 128-bit loads of the rows,
-// their neighbour rows and b.  The rows are taken in the children's order
-// (x fastest, then y, then z), so each coarse sum adds the same terms in the
-// same order as resid_restrict_kernel.
+// bc = 0.5 * sum over the 8 children of (bf - (sum_nbr(xf) - 6 xf)), a thread
+// per pair of coarse cells along x (the coarse edge is even: only levels of
+// edge > 32 are restricted here).  Their 16 fine children, 4 consecutive cells
+// in each of the 4 fine rows (j, k) in {2jc, 2jc+1} x {2kc, 2kc+1}, are read
+// with 128-bit loads of the rows, their neighbour rows and b, in the
+// children's order (x fastest, then y, then z).
 __global__ void __launch_bounds__(kMGThreads)
 resid_restrict2_kernel(const float *__restrict__ xf, const float *__restrict__ bf, float *__restrict__ bc,
                        int dc, int x_zero, int ldc) {
@@ -235,22 +141,9 @@ resid_restrict2_kernel(const float *__restrict__ xf, const float *__restrict__ b
         make_float2(s0 * 0.5f, s1 * 0.5f);
 }
 
-__global__ void __launch_bounds__(kMGThreads)
-prolong_kernel(float *__restrict__ xf, const float *__restrict__ xc, int df, int ldf) {
-    const uint32_t per = (uint32_t)df * df * df;
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= per) return;
-    const size_t comp = blockIdx.y;
-    const int dc = df >> 1;
-    int i, j, k;
-    split3(t, df, df, ldf, ldf, i, j, k);
-    xf[comp * per + t] += xc[comp * (size_t)dc * dc * dc + ((size_t)(k >> 1) * dc + (j >> 1)) * dc + (i >> 1)];
-}
-
-// The same prolongation by injection with a thread per group of 4 fine cells
-// of a row (fine edge a multiple of 4): one 128-bit read-modify-write of the
-// fine cells and the 2 coarse cells under them (each cell gets the same single
-// addition as in prolong_kernel).
+// Prolongation by injection with a thread per group of 4 fine cells of a row:
+// one 128-bit read-modify-write of the fine cells and the 2 coarse cells under
+// them (before the blocked smoother; the sweeps fold it into their reads).
 __global__ void __launch_bounds__(kMGThreads)
 prolong4_kernel(float *__restrict__ xf, const float *__restrict__ xc, int df, int ldf) {
     const int q = df >> 2;
@@ -296,48 +189,6 @@ __global__ void __launch_bounds__(512) coarse_kernel(float *__restrict__ x, cons
         double *tmp = cur; cur = nxt; nxt = tmp;
     }
     if (t < cells) x[comp * cells + t] = (float)cur[t];
-}
-
-// The coarsest solve always starts from x = 0 in the reference schedule at
-// two or more levels, so its 100 Jacobi sweeps are one fixed linear map
-// x = P b.  Column j of P is the sweep applied to the unit vector e_j (one
-// block per column); P is stored row-major [row][col].
-__global__ void __launch_bounds__(512) coarse_op_column_kernel(double *__restrict__ op, int d) {
-    __shared__ double xa[512], xb[512];
-    const int cells = d * d * d;
-    const int col = blockIdx.x;
-    const int t = threadIdx.x;
-    if (t < cells) xa[t] = 0.0;
-    __syncthreads();
-    const int i = t % d, j = (t / d) % d, k = t / (d * d);
-    double *cur = xa, *nxt = xb;
-    for (int it = 0; it < 100; it++) {
-        if (t < cells) {
-            double r = nb_sum64(cur, i, j, k, d, (size_t)t);
-            r -= (t == col) ? 1.0 : 0.0;
-            nxt[t] = r / 6;
-        }
-        __syncthreads();
-        double *tmp = cur; cur = nxt; nxt = tmp;
-    }
-    if (t < cells) op[(size_t)t * cells + col] = cur[t];
-}
-
-// x = P b per component: one warp per (row, component), lanes stride the row.
-__global__ void __launch_bounds__(256)
-coarse_apply_kernel(const double *__restrict__ op, float *__restrict__ x, const float *__restrict__ b, int cells,
-                    int comps) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= cells * comps) return;
-    const int row = warp % cells, comp = warp / cells;
-    const double *prow = op + (size_t)row * cells;
-    const float *bc = b + (size_t)comp * cells;
-    double acc = 0.0;
-    for (int c = lane; c < cells; c += 32) acc = fma(prow[c], (double)bc[c], acc);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) x[(size_t)comp * cells + row] = (float)acc;
 }
 
 // r = b - (sum_nbr(psi) - 6 psi) in FP64, stored as the FP32 right-hand side
@@ -392,26 +243,7 @@ __global__ void dc_update_kernel(double *__restrict__ psi, const float *__restri
 
 inline dim3 grid_for(uint32_t per, int comps) { return dim3((per + kMGThreads - 1) / kMGThreads, comps); }
 
-// Coarsest solve from x = 0: the precomputed operator when available, else
-// the sweeps themselves.
-void coarse_solve(const MGPlan &m) {
-    const Level &c = m.lv[m.levels - 1];
-    ::pppm::note_launch();
-    if (m.coarse_op && m.levels >= 2) {
-        const unsigned warps = c.cells * (unsigned)m.comps;
-        coarse_apply_kernel<<<(warps * 32 + 255) / 256, 256, 0, m.st>>>(m.coarse_op, c.x, c.b, (int)c.cells, m.comps);
-    } else {
-        coarse_kernel<<<m.comps, 512, 0, m.st>>>(c.x, c.b, (int)c.d);
-    }
-}
-
 }  // namespace
-
-cudaError_t build_coarse_operator(int d, double *op, cudaStream_t st) {
-    ::pppm::note_launch();
-    coarse_op_column_kernel<<<d * d * d, 512, 0, st>>>(op, d);
-    return cudaGetLastError();
-}
 
 int mg_level_count(uint32_t n) {
     // MG/MultiGrid.h:114-127
@@ -444,36 +276,25 @@ static bool tb_level(const MGPlan &m, int j) { return m.tb_var[j] >= 0 && m.lv[j
 
 static float *x_ptr(const MGPlan &m, int j, XAt at) { return at == kXAlt ? m.lv[j].x2 : m.lv[j].x; }
 
-// Four red-black iterations (8 half sweeps, odd cells first) at level j,
-// starting from `in` (zero, or x in one of the two copies) plus, when xc is
-// set, the injected coarse correction xc[parent] (the prolongation that
-// precedes the reference's post-smoothing).  Blocked levels run 8 / T passes
-// of the blocked smoother, ping-ponging between the two copies; the others run
-// the half sweeps in place on the main copy.  Returns where the result is:
-// a pre-smoothing from zero ends in the main copy for an even pass count and
-// in the second copy for an odd one, a post-smoothing from there always ends
-// in the main copy.
-// bc = the restricted residual of the level above (a pair of coarse cells per
-// thread where the coarse edge is even).
+// bc = the restricted residual of the level above.
 static void launch_restrict(const MGPlan &m, const float *xf, const float *bf, float *bc, int dc, int x_zero) {
-    if ((dc % 2) == 0)
-        resid_restrict2_kernel<<<grid_for((uint32_t)(dc / 2) * dc * dc, m.comps), kMGThreads, 0, m.st>>>(
-            xf, bf, bc, dc, x_zero, edge_log2(dc));
-    else
-        resid_restrict_kernel<<<grid_for((uint32_t)dc * dc * dc, m.comps), kMGThreads, 0, m.st>>>(
-            xf, bf, bc, dc, x_zero, edge_log2(dc));
+    resid_restrict2_kernel<<<grid_for((uint32_t)(dc / 2) * dc * dc, m.comps), kMGThreads, 0, m.st>>>(
+        xf, bf, bc, dc, x_zero, edge_log2(dc));
 }
 
-// x += the coarser level's xc injected (a group of 4 cells per thread where
-// the edge allows).
+// x += the coarser level's xc injected.
 static void launch_prolong(const MGPlan &m, float *x, const float *xc, int d) {
-    if ((d % 4) == 0)
-        prolong4_kernel<<<grid_for((uint32_t)(d / 4) * d * d, m.comps), kMGThreads, 0, m.st>>>(x, xc, d,
-                                                                                                edge_log2(d));
-    else
-        prolong_kernel<<<grid_for((uint32_t)d * d * d, m.comps), kMGThreads, 0, m.st>>>(x, xc, d, edge_log2(d));
+    prolong4_kernel<<<grid_for((uint32_t)(d / 4) * d * d, m.comps), kMGThreads, 0, m.st>>>(x, xc, d, edge_log2(d));
 }
 
+// Four red-black iterations (8 half sweeps, odd cells first) at level j of
+// edge > 32, starting from `in` (zero, or x in one of its copies) plus, when
+// xc is set, the injected coarse correction xc[parent] (the prolongation that
+// precedes the reference's post-smoothing).  Four passes of the sweep kernel,
+// through the scratch copy and back, each fusing both half sweeps; blocked
+// levels (opt-in) run 8 / T passes of the blocked smoother, ping-ponging
+// between their two copies.  Returns where the result is: the main copy, or
+// for a blocked pre-smoothing from zero with an odd pass count the second.
 static cudaError_t smooth(const MGPlan &m, int j, XAt in, const float *xc, XAt *out) {
     const Level &L = m.lv[j];
     const int d = (int)L.d;
@@ -502,51 +323,40 @@ static cudaError_t smooth(const MGPlan &m, int j, XAt in, const float *xc, XAt *
         *out = cur;
         return cudaSuccess;
     }
-    if (in == kXZero) PPPM_CUDA_TRY(cudaMemsetAsync(L.x, 0, sizeof(float) * m.comps * (size_t)L.cells, m.st));
-    if (xc) {
-        ::pppm::note_launch();
-        launch_prolong(m, L.x, xc, d);
-    }
-    if ((d % 4) == 0) {
-        const dim3 g = grid_for((uint32_t)(d / 4) * d * d, m.comps);
-        for (int it = 0; it < 4; it++) {
-            ::pppm::note_launch();
-            rbsor4_kernel<<<g, kMGThreads, 0, m.st>>>(L.x, L.b, d, 1, edge_log2(d));
-            ::pppm::note_launch();
-            rbsor4_kernel<<<g, kMGThreads, 0, m.st>>>(L.x, L.b, d, 0, edge_log2(d));
-        }
-    } else {
-        const dim3 g = grid_for((uint32_t)(d / 2) * d * d, m.comps);
-        for (int it = 0; it < 4; it++) {
-            ::pppm::note_launch();
-            rbsor_kernel<<<g, kMGThreads, 0, m.st>>>(L.x, L.b, d, 1, edge_log2(d));
-            ::pppm::note_launch();
-            rbsor_kernel<<<g, kMGThreads, 0, m.st>>>(L.x, L.b, d, 0, edge_log2(d));
-        }
+    // four sweeps ping-pong between x and the scratch copy and end in x
+    const float *src = in == kXZero ? nullptr : L.x;
+    for (int it = 0; it < 4; it++) {
+        float *dst = (it & 1) ? L.x : m.scratch;
+        PPPM_CUDA_TRY(mg_sweep(src, L.b, it == 0 ? xc : nullptr, dst, d, m.comps, m.st));
+        src = dst;
     }
     *out = kXMain;
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 // One FP32 V(4,4) cycle from level `level` down (MG/MultiGrid.cpp:128-201).
 // The cycle's x at `level` starts at zero plus, when xc is set, the injected
 // correction from level + 1 (the full multigrid's prolongation); the coarser
 // levels start at zero as the reference zeroes them.  The result is left in
-// lv[level].x.
+// lv[level].x.  The levels from mg_tail_level on run in one launch.
 static cudaError_t vcycle32(const MGPlan &m, int level, const float *xc = nullptr) {
-    const int L = m.levels;
+    // one level: the coarsest solve alone, from zero
+    if (m.levels - level == 1) {
+        const Level &c = m.lv[level];
+        PPPM_CUDA_TRY(cudaMemsetAsync(c.x, 0, sizeof(float) * m.comps * (size_t)c.cells, m.st));
+        ::pppm::note_launch();
+        coarse_kernel<<<m.comps, 512, 0, m.st>>>(c.x, c.b, (int)c.d);
+        return cudaGetLastError();
+    }
+    const int T = mg_tail_level(m);
     XAt at[kMaxLevels];
-    for (int j = level; j < L - 1; j++) {
+    for (int j = level; j < T; j++) {
         PPPM_CUDA_TRY(smooth(m, j, kXZero, j == level ? xc : nullptr, &at[j]));
         ::pppm::note_launch();
         launch_restrict(m, x_ptr(m, j, at[j]), m.lv[j].b, m.lv[j + 1].b, (int)m.lv[j + 1].d, 0);
     }
-    // the coarsest solve starts from zero (a cycle on the coarsest level alone
-    // included: it is only ever asked for from a zero start)
-    if (level == L - 1 || !m.coarse_op)
-        PPPM_CUDA_TRY(cudaMemsetAsync(m.lv[L - 1].x, 0, sizeof(float) * m.comps * (size_t)m.lv[L - 1].cells, m.st));
-    coarse_solve(m);
-    for (int j = L - 2; j >= level; j--) {
+    PPPM_CUDA_TRY(mg_tail_launch(m, std::max(T, level), false));
+    for (int j = T - 1; j >= level; j--) {
         XAt res;
         PPPM_CUDA_TRY(smooth(m, j, at[j], m.lv[j + 1].x, &res));
     }
@@ -557,15 +367,14 @@ static cudaError_t vcycle32(const MGPlan &m, int level, const float *xc = nullpt
 // (MG/MultiGrid.cpp:202-246; x = 0 on entry, so the residual chain is a
 // plain restriction of b).
 static cudaError_t fmg32(const MGPlan &m) {
-    const int L = m.levels;
-    for (int j = 0; j < L - 1; j++) {
+    if (m.levels == 1) return vcycle32(m, 0);
+    const int T = mg_tail_level(m);
+    for (int j = 0; j < T; j++) {
         ::pppm::note_launch();
         launch_restrict(m, m.lv[j].x, m.lv[j].b, m.lv[j + 1].b, (int)m.lv[j + 1].d, 1);
     }
-    PPPM_CUDA_TRY(cudaMemsetAsync(m.lv[L - 1].x, 0, sizeof(float) * m.comps * (size_t)m.lv[L - 1].cells, m.st));
-    coarse_solve(m);
-    PPPM_CUDA_TRY(cudaGetLastError());
-    for (int j = L - 2; j >= 0; j--) PPPM_CUDA_TRY(vcycle32(m, j, m.lv[j + 1].x));
+    PPPM_CUDA_TRY(mg_tail_launch(m, T, true));
+    for (int j = T - 1; j >= 0; j--) PPPM_CUDA_TRY(vcycle32(m, j, m.lv[j + 1].x));
     return cudaGetLastError();
 }
 
@@ -730,6 +539,7 @@ static cudaError_t tune_level(MGPlan &m, int j, int sms, int dev, int *best_out,
     for (int v = -1; v < nvar && e == cudaSuccess; v++) {
         MGPlan t = m;
         t.st = st;
+        t.scratch = L.x2;
         for (int q = 0; q < kMaxLevels; q++) t.tb_var[q] = -1;
         if (v >= 0) {
             int per_sm = 1;
@@ -784,11 +594,8 @@ cudaError_t mg_tb_setup(MGPlan &m, float *pool, int forced) {
         static std::once_flag once;
         static cudaError_t carve = cudaSuccess;
         std::call_once(once, [] {
-            const void *k[] = {(const void *)rbsor_kernel, (const void *)rbsor4_kernel,
-                               (const void *)prolong4_kernel, (const void *)resid_restrict_kernel,
-                               (const void *)resid_restrict2_kernel,
-                               (const void *)prolong_kernel, (const void *)dc_residual_kernel,
-                               (const void *)dc_update_kernel};
+            const void *k[] = {(const void *)prolong4_kernel, (const void *)resid_restrict2_kernel,
+                               (const void *)dc_residual_kernel, (const void *)dc_update_kernel};
             for (const void *f : k)
                 if (carve == cudaSuccess)
                     carve = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -892,7 +699,7 @@ static MGPlan scene_plan(pppm_scene *s) {
     m.vort = s->vort;
     m.P = s->dparams;
     m.norms = s->norms;
-    m.coarse_op = s->coarse_op;
+    m.scratch = s->far;  // written by the far-field kernel after every solve
     return m;
 }
 

@@ -100,7 +100,7 @@ struct MGPlan {
     const float *vort = nullptr;    // b = -(vort * h2f) from the P2M grid
     const DevParams *P = nullptr;
     double *norms = nullptr;        // [2] device scratch
-    const double *coarse_op = nullptr;  // [cells][cells] FP64 map b -> x of the coarsest solve, or null
+    float *scratch = nullptr;       // [comps][C0] second copy of a level's x while it is smoothed
 };
 
 // Every device and pinned-host allocation of the library goes through these
@@ -109,7 +109,35 @@ struct MGPlan {
 cudaError_t device_malloc(void **p, size_t bytes);
 cudaError_t host_malloc(void **p, size_t bytes);
 
-cudaError_t build_coarse_operator(int d, double *op, cudaStream_t st);
+#ifdef __CUDACC__
+// The red-black SOR update of one cell from its neighbour sum and right-hand
+// side (MG/MultiGrid_kernel.cu:766, omega = 1.43f, 1 - omega formed in
+// float), one expression for every smoother kernel so that they round alike.
+constexpr float kOmegaF = 1.43f;
+constexpr float kOneMinusOmegaF = 1.0f - 1.43f;
+__device__ __forceinline__ float mg_sor_update(float x, float nb, float b) {
+    const float r = nb - b;
+    return kOneMinusOmegaF * x + (kOmegaF * r) * (1.0f / 6.0f);
+}
+#endif
+
+// The launch that runs a hierarchy's small levels (mg_tail.cu): edges of its
+// levels (dA = 0: the top is level B), the top level's x and b, and the
+// coarsest level's one-dimensional eigenbasis [mode][cell] and eigenvalues.
+struct TailArgs {
+    int dA = 0, dB = 0, dC = 0;
+    float *x = nullptr;
+    const float *b = nullptr;
+    double basis[64] = {};
+    double lambda[8] = {};
+};
+int mg_tail_level(const MGPlan &m);
+cudaError_t mg_tail_prepare();
+cudaError_t mg_tail_launch(const MGPlan &m, int level, bool fmg);
+// One red-black sweep of a level of edge > 32 (mg_sweep.cu).
+cudaError_t mg_sweep_prepare();
+cudaError_t mg_sweep(const float *x, const float *b, const float *xc, float *out, int d, int comps, cudaStream_t st);
+
 cudaError_t mg_capture_graph(const MGPlan &m, cudaGraphExec_t *exec, unsigned *kernel_nodes);
 
 // Density grid and heat-particle hash of the buoyancy source (buoyancy.cu),
@@ -163,7 +191,6 @@ struct pppm_scene {
     double *psi = nullptr;                // [3][C]
     float *far = nullptr;                 // [3][C]
     double *norms = nullptr;              // [2] residual / rhs squared norms
-    double *coarse_op = nullptr;          // coarsest-level operator (levels >= 2)
     cudaGraphExec_t mg_graph = nullptr;   // reference-schedule solve, captured once
     unsigned mg_graph_kernels = 0;
     float *mg_x2_pool = nullptr;          // second x copies of the blocked-smoother levels

@@ -1,0 +1,49 @@
+"""The multigrid's level kernels at the edges where they change: the launch
+that holds the levels of edge <= 32 (csrc/mg_tail.cu: slabs of 4 planes of a
+level of edge 17 to 32, the level of edge 9 to 16 and the coarsest one), and
+the fused red-black sweep of the larger levels (csrc/mg_sweep.cu: whole rows,
+tiles of at most 16 of them, chunks of planes), against the oracle's FP64
+schedule.
+
+A solve ends with an FP64 defect correction whose FP32 cycle rounds relative
+to the correction it computes: below 1e-6 of the solution (the bound of the
+scene's potential in test_gpu_parity).  One V-cycle from a random x is all
+correction, a sum of eight half sweeps a level and their transfers, each
+rounding to 2^-24 of values of the correction's size: 16 half sweeps, both
+transfers and five levels stay below 100 x 2^-24 = 6e-6 of it.
+"""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def pb():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import pppm_vortex_bouyant_flow_sample_b200 as pb
+    pb.load()
+    return pb
+
+
+@pytest.mark.parametrize("n", [10, 12, 14, 16, 20, 24, 28, 32, 40, 48, 56, 64, 80, 112, 160])
+def test_full_multigrid_and_vcycle(pb, oracle, n):
+    import torch
+    rng = np.random.default_rng(n)
+    b = rng.standard_normal(n ** 3)
+    mg = pb.MultiGridSolver3DPeriod_double()
+    mg.m_InitialSystem(n, n, n)
+    x = torch.zeros(n ** 3, dtype=torch.float64, device="cuda")
+    mg.m_FullMultiGrid(x, torch.from_numpy(b).cuda())
+    ref = oracle.mg_fmg(np.zeros(n ** 3), b, n)
+    assert rel_l2(x.cpu().numpy(), ref) <= 1e-6
+    x0 = rng.standard_normal(n ** 3)
+    x = torch.from_numpy(x0.copy()).cuda()
+    mg.m_Vcycle(x, torch.from_numpy(b).cuda())
+    ref = oracle.mg_vcycle(x0, b, n)
+    assert np.linalg.norm(x.cpu().numpy() - ref) <= 6e-6 * np.linalg.norm(ref - x0)
+    mg.m_FinalMemoryEachLevel()
