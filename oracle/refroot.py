@@ -3,14 +3,17 @@
 The checker libraries under oracle/_ref are compiled from the reference's own
 sources where they lie.  Their location comes from the environment variable
 PPPM_REFERENCE_ROOT, else from the "reference_path" entry of the repository's
-BASELINE.json; with neither (or a path that does not exist, as on a host that
-only runs the prebuilt checkers) there is nothing to build.
+BASELINE.json; with neither (or a path that does not exist or does not hold the
+sources, as on a host that only runs the prebuilt checkers) there is nothing to
+build.
 """
 from __future__ import annotations
 
 import json
 import os
 
+# directories of the sources that the checkers are compiled from
+_PARTS = ("hybridFastSummation", "particle_hash", "multigrid", "Particle_renderer")
 _REPO = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
@@ -23,4 +26,6 @@ def reference_root():
                 cand = json.load(f).get("reference_path")
         except (OSError, ValueError):
             cand = None
-    return cand if cand and os.path.isdir(cand) else None
+    if not cand or not all(os.path.isdir(os.path.join(cand, d)) for d in _PARTS):
+        return None
+    return cand
