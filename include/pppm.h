@@ -243,7 +243,7 @@ uint64_t pppm_kernel_launches(void);
 /* The multigrid smoother's autotuner (no reference counterpart).  By default
  * every level runs the plain red-black half sweeps.  With PPPM_MG_TB=auto in
  * the environment when a scene or multigrid object is created, each level of
- * edge >= 256 runs either the plain half sweeps or one of the temporally
+ * edge >= 256 runs either the sweep kernel or one of the temporally
  * blocked variants (T half sweeps per pass, TX x TY tiles, TMA plane
  * staging), whichever measured fastest for that edge and component count on
  * this device; PPPM_MG_TB=<index> forces one variant.  Every choice gives the

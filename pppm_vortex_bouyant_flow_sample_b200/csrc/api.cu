@@ -243,6 +243,8 @@ cudaError_t alloc_grid_side(pppm_scene *s) {
     PPPM_CUDA_TRY(cudaMemset(s->mflag, 0, sizeof(uint32_t) * s->C));
     PPPM_CUDA_TRY(dalloc(&s->dparams, 1));
     PPPM_CUDA_TRY(dalloc(&s->norms, 2));
+    if (s->prm.mg_mode == PPPM_MG_CONVERGED)
+        PPPM_CUDA_TRY(::pppm::host_malloc((void **)&s->norms_h, 2 * sizeof(double)));
     PPPM_CUDA_TRY(dalloc(&s->pair_count, 1));
     // initialise on a private stream (no device-wide synchronisation)
     cudaStream_t st = nullptr;
@@ -277,6 +279,7 @@ void destroy_scene(pppm_scene *s) {
     cudaFree(s->sub_end);
     cudaFree(s->dparams);
     cudaFree(s->norms);
+    if (s->norms_h) cudaFreeHost(s->norms_h);
     cudaFree(s->pair_count);
     if (s->mg_graph) cudaGraphExecDestroy(s->mg_graph);
     pppm::free_buoyancy(s->buoy);

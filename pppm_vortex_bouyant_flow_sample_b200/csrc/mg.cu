@@ -23,6 +23,9 @@
 // Levels of edge > 32 run one kernel per red-black sweep (mg_sweep.cu); the
 // restriction takes a pair of coarse cells per thread with 128-bit loads.  The
 // temporally blocked smoother of mg_tb.cu is opt-in (PPPM_MG_TB).
+//
+// The solve to a tolerance (CONVERGED) takes its own cycles, see
+// corrected_cycle; the fixed schedule keeps the one above.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -38,16 +41,7 @@ namespace {
 
 constexpr int kMGThreads = 256;
 
-__device__ __forceinline__ float nb_sum(const float *__restrict__ x, int i, int j, int k, int d, size_t c) {
-    const size_t dd = (size_t)d * d;
-    const float lv = (i > 0) ? x[c - 1] : 0.f;
-    const float rv = (i < d - 1) ? x[c + 1] : 0.f;
-    const float uv = (j < d - 1) ? x[c + d] : 0.f;
-    const float dv = (j > 0) ? x[c - d] : 0.f;
-    const float fv = (k > 0) ? x[c - dd] : 0.f;
-    const float bv = (k < d - 1) ? x[c + dd] : 0.f;
-    return ((lv + rv) + (uv + dv)) + (fv + bv);
-}
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 
 __device__ __forceinline__ double nb_sum64(const double *__restrict__ x, int i, int j, int k, int d, size_t c) {
     const size_t dd = (size_t)d * d;
@@ -83,8 +77,6 @@ __device__ __forceinline__ void split3(uint32_t t, int a, int d, int la, int ld,
     }
 }
 
-__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
-
 // Residual at the fine level restricted to the coarse level in one pass:
 // bc = 0.5 * sum over the 8 children of (bf - (sum_nbr(xf) - 6 xf)), a thread
 // per pair of coarse cells along x (the coarse edge is even: only levels of
@@ -92,9 +84,12 @@ __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast
 // in each of the 4 fine rows (j, k) in {2jc, 2jc+1} x {2kc, 2kc+1}, are read
 // with 128-bit loads of the rows, their neighbour rows and b, in the
 // children's order (x fastest, then y, then z).
+// CORR: the corrected cycle's diagonal, 6 less the level's ghost factor per
+// boundary face.
+template <bool CORR>
 __global__ void __launch_bounds__(kMGThreads)
 resid_restrict2_kernel(const float *__restrict__ xf, const float *__restrict__ bf, float *__restrict__ bc,
-                       int dc, int x_zero, int ldc) {
+                       int dc, int x_zero, int ldc, float ghost) {
     const int h = dc >> 1;  // coarse pairs per row
     const uint32_t per2 = (uint32_t)h * dc * dc;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -129,7 +124,11 @@ resid_restrict2_kernel(const float *__restrict__ xf, const float *__restrict__ b
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 const float nb = ((xs[e] + xs[e + 2]) + (us[e] + ds[e])) + (fs[e] + bs[e]);
-                r[e] -= nb - 6.f * xs[e + 1];
+                float diag = 6.f;
+                if (CORR)
+                    diag -= ghost * (float)((j == 0) + (j == df - 1) + (k == 0) + (k == df - 1) + (i0 + e == 0) +
+                                            (i0 + e == df - 1));
+                r[e] -= nb - diag * xs[e + 1];
             }
         }
         s0 += r[0];
@@ -193,28 +192,72 @@ __global__ void __launch_bounds__(512) coarse_kernel(float *__restrict__ x, cons
 
 // r = b - (sum_nbr(psi) - 6 psi) in FP64, stored as the FP32 right-hand side
 // of the correction equation.  b is read from b64 (FP64) or formed as
-// -(vort * h2f) from the FP32 P2M grid.  Optional squared norms of r and b.
+// -(vort * h2f) from the FP32 P2M grid.  Optional squared norms of r and b:
+// each block adds its sums once over all the groups it takes.  W = 4: a thread
+// takes groups of 4 cells of a row (edge a multiple of 4) with 128-bit loads.
+template <int W>
 __global__ void __launch_bounds__(kMGThreads)
 dc_residual_kernel(const double *__restrict__ psi, const double *__restrict__ b64, const float *__restrict__ vort,
                    const DevParams *__restrict__ P, float *__restrict__ rout, int d, int ld,
                    double *__restrict__ norms) {
-    const uint32_t per = (uint32_t)d * d * d;
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t comp = blockIdx.y;
+    const int q = d / W;
+    const uint32_t per = (uint32_t)q * d * d;
+    const size_t comp = blockIdx.y, cells = (size_t)d * d * d, dd = (size_t)d * d;
+    const double *x = psi + comp * cells;
+    const float h2f = b64 ? 0.f : P->h2f;
     double r2 = 0.0, b2 = 0.0;
-    if (t < per) {
-        const double *x = psi + comp * per;
-        int i, j, k;
-        split3(t, d, d, ld, ld, i, j, k);
-        double bv;
-        if (b64)
-            bv = b64[comp * per + t];
-        else
-            bv = (double)(-(vort[comp * per + t] * P->h2f));
-        const double r = bv - (nb_sum64(x, i, j, k, d, t) - 6.0 * x[t]);
-        rout[comp * per + t] = (float)r;
-        r2 = r * r;
-        b2 = bv * bv;
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < per; t += gridDim.x * blockDim.x) {
+        int g, j, k;
+        split3(t, q, d, ld >= 2 ? ld - (W == 4 ? 2 : 0) : -1, ld >= 2 ? ld : -1, g, j, k);
+        const int i0 = W * g;
+        const size_t c = ((size_t)k * d + j) * d + i0;
+        auto row = [&](size_t at, bool in, double (&v)[W]) {
+            if constexpr (W == 4) {
+                const double2 z = make_double2(0.0, 0.0);
+                const double2 a = in ? *reinterpret_cast<const double2 *>(x + at) : z;
+                const double2 b = in ? *reinterpret_cast<const double2 *>(x + at + 2) : z;
+                v[0] = a.x;
+                v[1] = a.y;
+                v[2] = b.x;
+                v[3] = b.y;
+            } else {
+                v[0] = in ? x[at] : 0.0;
+            }
+        };
+        double v[W], up[W], dn[W], fr[W], bk[W], xs[W + 2];
+        row(c, true, v);
+        row(c + d, j < d - 1, up);
+        row(c - d, j > 0, dn);
+        row(c - dd, k > 0, fr);
+        row(c + dd, k < d - 1, bk);
+        xs[0] = i0 > 0 ? x[c - 1] : 0.0;
+        xs[W + 1] = i0 + W < d ? x[c + W] : 0.0;
+#pragma unroll
+        for (int e = 0; e < W; e++) xs[e + 1] = v[e];
+        double bv[W];
+        if (b64) {
+#pragma unroll
+            for (int e = 0; e < W; e++) bv[e] = b64[comp * cells + c + e];
+        } else if constexpr (W == 4) {
+            const float4 w = ld4(vort + comp * cells + c);
+            bv[0] = (double)(-(w.x * h2f));
+            bv[1] = (double)(-(w.y * h2f));
+            bv[2] = (double)(-(w.z * h2f));
+            bv[3] = (double)(-(w.w * h2f));
+        } else {
+            bv[0] = (double)(-(vort[comp * cells + c] * h2f));
+        }
+        float ro[W];
+#pragma unroll
+        for (int e = 0; e < W; e++) {
+            const double nb = ((xs[e] + xs[e + 2]) + (up[e] + dn[e])) + (fr[e] + bk[e]);
+            const double r = bv[e] - (nb - 6.0 * v[e]);
+            ro[e] = (float)r;
+            r2 += r * r;
+            b2 += bv[e] * bv[e];
+        }
+        if constexpr (W == 4) *reinterpret_cast<float4 *>(rout + comp * cells + c) = make_float4(ro[0], ro[1], ro[2], ro[3]);
+        else rout[comp * cells + c] = ro[0];
     }
     if (norms) {
 #pragma unroll
@@ -277,9 +320,13 @@ static bool tb_level(const MGPlan &m, int j) { return m.tb_var[j] >= 0 && m.lv[j
 static float *x_ptr(const MGPlan &m, int j, XAt at) { return at == kXAlt ? m.lv[j].x2 : m.lv[j].x; }
 
 // bc = the restricted residual of the level above.
-static void launch_restrict(const MGPlan &m, const float *xf, const float *bf, float *bc, int dc, int x_zero) {
-    resid_restrict2_kernel<<<grid_for((uint32_t)(dc / 2) * dc * dc, m.comps), kMGThreads, 0, m.st>>>(
-        xf, bf, bc, dc, x_zero, edge_log2(dc));
+static void launch_restrict(const MGPlan &m, const float *xf, const float *bf, float *bc, int dc, int x_zero,
+                            float ghost = 0.f) {
+    const dim3 g = grid_for((uint32_t)(dc / 2) * dc * dc, m.comps);
+    if (ghost == 0.f)
+        resid_restrict2_kernel<false><<<g, kMGThreads, 0, m.st>>>(xf, bf, bc, dc, x_zero, edge_log2(dc), 0.f);
+    else
+        resid_restrict2_kernel<true><<<g, kMGThreads, 0, m.st>>>(xf, bf, bc, dc, x_zero, edge_log2(dc), ghost);
 }
 
 // x += the coarser level's xc injected.
@@ -295,7 +342,10 @@ static void launch_prolong(const MGPlan &m, float *x, const float *xc, int d) {
 // levels (opt-in) run 8 / T passes of the blocked smoother, ping-ponging
 // between their two copies.  Returns where the result is: the main copy, or
 // for a blocked pre-smoothing from zero with an odd pass count the second.
-static cudaError_t smooth(const MGPlan &m, int j, XAt in, const float *xc, XAt *out) {
+// With psi the result of the last sweep is added to it (or becomes it) and is
+// not stored elsewhere.
+static cudaError_t smooth(const MGPlan &m, int j, XAt in, const float *xc, XAt *out, double *psi = nullptr,
+                          bool set_psi = false) {
     const Level &L = m.lv[j];
     const int d = (int)L.d;
     if (tb_level(m, j)) {
@@ -324,29 +374,49 @@ static cudaError_t smooth(const MGPlan &m, int j, XAt in, const float *xc, XAt *
         return cudaSuccess;
     }
     // four sweeps ping-pong between x and the scratch copy and end in x
-    const float *src = in == kXZero ? nullptr : L.x;
+    SweepSpec sp;
+    sp.x = in == kXZero ? nullptr : L.x;
+    sp.b = L.b;
+    sp.d = d;
+    sp.comps = m.comps;
     for (int it = 0; it < 4; it++) {
-        float *dst = (it & 1) ? L.x : m.scratch;
-        PPPM_CUDA_TRY(mg_sweep(src, L.b, it == 0 ? xc : nullptr, dst, d, m.comps, m.st));
-        src = dst;
+        sp.xc = it == 0 ? xc : nullptr;
+        sp.out = (it & 1) ? L.x : m.scratch;
+        if (it == 3 && psi) {
+            sp.psi = psi;
+            sp.set_psi = set_psi;
+        }
+        PPPM_CUDA_TRY(mg_sweep(sp, m.st));
+        sp.x = sp.out;
     }
     *out = kXMain;
     return cudaSuccess;
+}
+
+// psi += x (or psi = x) of the finest level.
+static cudaError_t add_to_psi(const MGPlan &m, double *psi, bool set_psi) {
+    const size_t cnt = (size_t)m.comps * m.lv[0].cells;
+    ::pppm::note_launch();
+    dc_update_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, m.st>>>(psi, m.lv[0].x, cnt, set_psi ? 1 : 0);
+    return cudaGetLastError();
 }
 
 // One FP32 V(4,4) cycle from level `level` down (MG/MultiGrid.cpp:128-201).
 // The cycle's x at `level` starts at zero plus, when xc is set, the injected
 // correction from level + 1 (the full multigrid's prolongation); the coarser
 // levels start at zero as the reference zeroes them.  The result is left in
-// lv[level].x.  The levels from mg_tail_level on run in one launch.
-static cudaError_t vcycle32(const MGPlan &m, int level, const float *xc = nullptr) {
+// lv[level].x, or with psi (level 0) added to it or stored in it instead.  The
+// levels from mg_tail_level on run in one launch.
+static cudaError_t vcycle32(const MGPlan &m, int level, const float *xc = nullptr, double *psi = nullptr,
+                            bool set_psi = false) {
     // one level: the coarsest solve alone, from zero
     if (m.levels - level == 1) {
         const Level &c = m.lv[level];
         PPPM_CUDA_TRY(cudaMemsetAsync(c.x, 0, sizeof(float) * m.comps * (size_t)c.cells, m.st));
         ::pppm::note_launch();
         coarse_kernel<<<m.comps, 512, 0, m.st>>>(c.x, c.b, (int)c.d);
-        return cudaGetLastError();
+        PPPM_CUDA_TRY(cudaGetLastError());
+        return psi ? add_to_psi(m, psi, set_psi) : cudaSuccess;
     }
     const int T = mg_tail_level(m);
     XAt at[kMaxLevels];
@@ -355,27 +425,87 @@ static cudaError_t vcycle32(const MGPlan &m, int level, const float *xc = nullpt
         ::pppm::note_launch();
         launch_restrict(m, x_ptr(m, j, at[j]), m.lv[j].b, m.lv[j + 1].b, (int)m.lv[j + 1].d, 0);
     }
-    PPPM_CUDA_TRY(mg_tail_launch(m, std::max(T, level), false));
+    PPPM_CUDA_TRY(mg_tail_launch(m, std::max(T, level), kTailCycle));
     for (int j = T - 1; j >= level; j--) {
+        const bool last = j == 0 && psi && !tb_level(m, j);
         XAt res;
-        PPPM_CUDA_TRY(smooth(m, j, at[j], m.lv[j + 1].x, &res));
+        PPPM_CUDA_TRY(smooth(m, j, at[j], m.lv[j + 1].x, &res, last ? psi : nullptr, set_psi));
+        if (last) return cudaSuccess;
     }
-    return cudaGetLastError();
+    return psi ? add_to_psi(m, psi, set_psi) : cudaSuccess;
 }
 
-// Full multigrid in FP32 with lv[0].b holding the right-hand side
+// Ghost factor of a level of the corrected cycle (below): the zero of the
+// finest level's ghost cell lies half a fine cell beyond its boundary cells'
+// faces, 1/2 + 1/2^(level + 1) of level's own cells from their centres; the
+// line through it and a boundary cell's value is this multiple of that value
+// one cell further out.  0 on the finest level.
+float mg_ghost_factor(int level) {
+    const double delta = 0.5 + 0.5 / (double)(1 << level);
+    return (float)(1.0 - 1.0 / delta);
+}
+
+// One corrected cycle on lv[0].b from zero into psi, for the solve to a
+// tolerance, which is free to choose its iteration.  The reference's cycle
+// converges by about 0.3 a cycle of eight sweeps a level: its coarse levels
+// put the zero of the ghost cells a coarse cell beyond the boundary cells'
+// centres, where the fine level has it nearer (mg_ghost_factor), so the
+// correction is wrong along the faces, and injection is a poor interpolation.
+// With the coarse levels' zero at the fine one's place, trilinear
+// interpolation and omega = 1.25, V(2,2) converges by 0.02 a cycle of four
+// sweeps (64^3, 96^3: 0.016 and 0.017; omega 1.15: 0.046, 1.43: 0.05 and
+// above; injection: 0.07), independent of the edge.
+static cudaError_t corrected_cycle(const MGPlan &m, bool set_psi) {
+    const int T = mg_tail_level(m);
+    SweepSpec sp;
+    sp.comps = m.comps;
+    for (int j = 0; j < T; j++) {
+        const Level &L = m.lv[j];
+        sp.b = L.b;
+        sp.d = (int)L.d;
+        sp.corrected = j;
+        for (int it = 0; it < 2; it++) {
+            sp.x = it ? m.scratch : nullptr;
+            sp.out = it ? L.x : m.scratch;
+            PPPM_CUDA_TRY(mg_sweep(sp, m.st));
+        }
+        ::pppm::note_launch();
+        launch_restrict(m, L.x, L.b, m.lv[j + 1].b, (int)m.lv[j + 1].d, 0, mg_ghost_factor(j));
+    }
+    PPPM_CUDA_TRY(mg_tail_launch(m, T, kTailCorrected));
+    for (int j = T - 1; j >= 0; j--) {
+        const Level &L = m.lv[j];
+        sp.b = L.b;
+        sp.d = (int)L.d;
+        sp.corrected = j;
+        for (int it = 0; it < 2; it++) {
+            sp.x = it ? m.scratch : L.x;
+            sp.xc = it ? nullptr : m.lv[j + 1].x;
+            sp.out = it ? L.x : m.scratch;
+            if (it && j == 0) {
+                sp.psi = m.psi;
+                sp.set_psi = set_psi;
+            }
+            PPPM_CUDA_TRY(mg_sweep(sp, m.st));
+        }
+    }
+    return T == 0 ? add_to_psi(m, m.psi, set_psi) : cudaGetLastError();
+}
+
+// psi = the full multigrid in FP32 of the right-hand side in lv[0].b
 // (MG/MultiGrid.cpp:202-246; x = 0 on entry, so the residual chain is a
 // plain restriction of b).
 static cudaError_t fmg32(const MGPlan &m) {
-    if (m.levels == 1) return vcycle32(m, 0);
+    if (m.levels == 1) return vcycle32(m, 0, nullptr, m.psi, true);
     const int T = mg_tail_level(m);
     for (int j = 0; j < T; j++) {
         ::pppm::note_launch();
         launch_restrict(m, m.lv[j].x, m.lv[j].b, m.lv[j + 1].b, (int)m.lv[j + 1].d, 1);
     }
-    PPPM_CUDA_TRY(mg_tail_launch(m, T, true));
-    for (int j = T - 1; j >= 0; j--) PPPM_CUDA_TRY(vcycle32(m, j, m.lv[j + 1].x));
-    return cudaGetLastError();
+    PPPM_CUDA_TRY(mg_tail_launch(m, T, kTailFull));
+    for (int j = T - 1; j >= 0; j--)
+        PPPM_CUDA_TRY(vcycle32(m, j, m.lv[j + 1].x, j == 0 ? m.psi : nullptr, true));
+    return T == 0 ? add_to_psi(m, m.psi, true) : cudaSuccess;
 }
 
 // FP64 residual of the current psi, stored as the FP32 right-hand side of the
@@ -384,19 +514,11 @@ static cudaError_t dc_residual(const MGPlan &m, bool want_norms) {
     const uint32_t C0 = m.lv[0].cells;
     if (want_norms) PPPM_CUDA_TRY(cudaMemsetAsync(m.norms, 0, 2 * sizeof(double), m.st));
     ::pppm::note_launch();
-    dc_residual_kernel<<<grid_for(C0, m.comps), kMGThreads, 0, m.st>>>(m.psi, m.b64, m.vort, m.P, m.lv[0].b,
-                                                                       (int)m.lv[0].d, edge_log2((int)m.lv[0].d),
-                                                                       want_norms ? m.norms : nullptr);
-    return cudaGetLastError();
-}
-
-// e = V32(0, r); psi += e.
-static cudaError_t dc_correct(const MGPlan &m) {
-    const uint32_t C0 = m.lv[0].cells;
-    PPPM_CUDA_TRY(vcycle32(m, 0));
-    const size_t cnt = (size_t)m.comps * C0;
-    ::pppm::note_launch();
-    dc_update_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, m.st>>>(m.psi, m.lv[0].x, cnt, 0);
+    const int d = (int)m.lv[0].d, W = d % 4 == 0 ? 4 : 1;
+    dim3 g = grid_for(C0 / W, m.comps);
+    if (want_norms) g.x = std::min(g.x, 148u * 8u);
+    auto *k = W == 4 ? dc_residual_kernel<4> : dc_residual_kernel<1>;
+    k<<<g, kMGThreads, 0, m.st>>>(m.psi, m.b64, m.vort, m.P, m.lv[0].b, d, edge_log2(d), want_norms ? m.norms : nullptr);
     return cudaGetLastError();
 }
 
@@ -404,43 +526,42 @@ static cudaError_t dc_correct(const MGPlan &m) {
 // lv[0].b already holds r = b - A x64 (FP32), then e = V32(0, r) and
 // x64 += e — the reference's m_Vcycle(x, b) in exact arithmetic, the V-cycle
 // being a consistent linear iteration (MG/MultiGrid.cpp:128-201).
-cudaError_t mg_vcycle_update(const MGPlan &m, double *x64) {
-    const uint32_t C0 = m.lv[0].cells;
-    PPPM_CUDA_TRY(vcycle32(m, 0));
-    const size_t cnt = (size_t)m.comps * C0;
-    ::pppm::note_launch();
-    dc_update_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, m.st>>>(x64, m.lv[0].x, cnt, 0);
-    return cudaGetLastError();
-}
+cudaError_t mg_vcycle_update(const MGPlan &m, double *x64) { return vcycle32(m, 0, nullptr, x64, false); }
 
 static cudaError_t read_relres(const MGPlan &m, double *relres) {
-    double h[2];
-    PPPM_CUDA_TRY(cudaMemcpyAsync(h, m.norms, sizeof(h), cudaMemcpyDeviceToHost, m.st));
+    double own[2];
+    double *h = m.norms_h ? m.norms_h : own;
+    PPPM_CUDA_TRY(cudaMemcpyAsync(h, m.norms, 2 * sizeof(double), cudaMemcpyDeviceToHost, m.st));
     PPPM_CUDA_TRY(cudaStreamSynchronize(m.st));
     *relres = h[1] > 0 ? std::sqrt(h[0] / h[1]) : 0.0;
     return cudaSuccess;
 }
 
-// Whole solve: FMG in FP32, psi = x0, then the reference's final V-cycle as
-// an FP64 defect correction (this completes m_FullMultiGrid; cycles = 1).
-// CONVERGED then adds correction cycles while ||r||/||b|| > tol and
-// cycles < max_cycles, and reports the relative residual of the final psi.
+// Whole solve.  REFERENCE: psi = the FP32 full multigrid, then the reference's
+// final V-cycle as an FP64 defect correction (m_FullMultiGrid; cycles = 1).
+// CONVERGED: corrected cycles, each an FP64 defect correction, while
+// ||r||/||b|| > tol and cycles < max_cycles, the relative residual of the
+// final psi reported; the first two, which reach what the full multigrid and
+// its V-cycle reach, count as one (a hierarchy of one level iterates its
+// coarsest solve instead).  A residual just below tol gets one cycle more:
+// the reference's cycle gained a factor 4 and stopped at 0.4 tol on average,
+// this one gains 50.
 cudaError_t mg_solve(const MGPlan &m, int mode, double tol, int max_cycles, int *cycles_out, double *relres_out) {
-    PPPM_CUDA_TRY(fmg32(m));
-    const size_t cnt = (size_t)m.comps * m.lv[0].cells;
-    ::pppm::note_launch();
-    dc_update_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, m.st>>>(m.psi, m.lv[0].x, cnt, 1);
-    PPPM_CUDA_TRY(cudaGetLastError());
+    const bool corrected = mode == PPPM_MG_CONVERGED && m.levels > 1;
+    auto correct = [&]() { return corrected ? corrected_cycle(m, false) : vcycle32(m, 0, nullptr, m.psi, false); };
+    PPPM_CUDA_TRY(corrected ? corrected_cycle(m, true) : fmg32(m));
     PPPM_CUDA_TRY(dc_residual(m, false));
-    PPPM_CUDA_TRY(dc_correct(m));
+    PPPM_CUDA_TRY(correct());
     int cycles = 1;
     double rel = -1.0;
+    bool polished = false;
     if (mode == PPPM_MG_CONVERGED) {
         for (;;) {
             PPPM_CUDA_TRY(dc_residual(m, true));
             PPPM_CUDA_TRY(read_relres(m, &rel));
-            if (!(rel > tol) || cycles >= max_cycles) break;
-            PPPM_CUDA_TRY(dc_correct(m));
+            if (cycles >= max_cycles || !(rel > (corrected && !polished ? 0.2 * tol : tol))) break;
+            polished = polished || !(rel > tol);
+            PPPM_CUDA_TRY(correct());
             cycles++;
         }
     }
@@ -501,8 +622,8 @@ static int pick_zchunk(int d, int comps, int variant, int sms, int per_sm) {
 }
 
 namespace {
-// Autotuner results: fastest smoother (variant, or -1 for the plain half
-// sweeps) per (device, level edge, components), measured once per process.
+// Autotuner results: fastest smoother (variant, or -1 for the sweep
+// kernel) per (device, level edge, components), measured once per process.
 struct TuneKey {
     int dev, d, comps;
     bool operator==(const TuneKey &o) const { return dev == o.dev && d == o.d && comps == o.comps; }
@@ -517,9 +638,9 @@ TuneEntry g_tune[64];
 int g_tune_count = 0;
 }  // namespace
 
-// Times 8 half sweeps (four red-black iterations) of level j with the plain
-// kernels and with every blocked variant, on the level's own buffers (zeroed
-// first), and returns the fastest.  Every candidate computes the same values
+// Times 8 half sweeps (four red-black iterations) of level j with the
+// sweep kernel and with every blocked variant, on the level's own buffers
+// (zeroed first), and returns the fastest.  Every candidate computes the same values
 // bit for bit, so the choice only changes the time.
 static cudaError_t tune_level(MGPlan &m, int j, int sms, int dev, int *best_out, float *ms_out) {
     Level &L = m.lv[j];
@@ -579,7 +700,7 @@ static cudaError_t tune_level(MGPlan &m, int j, int sms, int dev, int *best_out,
 }
 
 // Points each qualifying level's x2 into `pool` (mg_tb_extra_floats floats),
-// picks its smoother — `forced` (a variant, or -1 for the plain half sweeps)
+// picks its smoother — `forced` (a variant, or -1 for the sweep kernel)
 // when >= -1, else the autotuner's choice — and builds its tensor maps and
 // z-chunk.
 cudaError_t mg_tb_setup(MGPlan &m, float *pool, int forced) {
@@ -594,8 +715,8 @@ cudaError_t mg_tb_setup(MGPlan &m, float *pool, int forced) {
         static std::once_flag once;
         static cudaError_t carve = cudaSuccess;
         std::call_once(once, [] {
-            const void *k[] = {(const void *)prolong4_kernel, (const void *)resid_restrict2_kernel,
-                               (const void *)dc_residual_kernel, (const void *)dc_update_kernel};
+            const void *k[] = {(const void *)prolong4_kernel, (const void *)resid_restrict2_kernel<false>,
+                               (const void *)dc_residual_kernel<4>, (const void *)dc_update_kernel};
             for (const void *f : k)
                 if (carve == cudaSuccess)
                     carve = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -672,11 +793,10 @@ size_t mg_tune_report(char *buf, size_t cap) {
     return w < cap ? w : cap;
 }
 
-// The plain half sweeps (rbsor4_kernel) measured faster inside a whole solve
-// than every blocked variant at 96^3 to 256^3 (256^3: 5.67 ms against 5.85 ms
-// with the autotuner's pick), and once a blocked pass has run, its large
-// shared-memory split slows the plain stencil kernels that follow.  So the
-// plain sweeps are the default; PPPM_MG_TB=auto runs the autotuner, an index
+// The sweep kernel (mg_sweep.cu) is faster than every blocked variant: 0.42 ms
+// for 8 half sweeps at 256^3 with three components against 0.81 ms for the best
+// of them (T2 128x32), which had lost inside a whole solve to two one-colour
+// passes a sweep already.  So it is the default; PPPM_MG_TB=auto runs the autotuner, an index
 // forces a variant.
 int mg_tb_default_variant() {
     const char *e = getenv("PPPM_MG_TB");
@@ -699,6 +819,7 @@ static MGPlan scene_plan(pppm_scene *s) {
     m.vort = s->vort;
     m.P = s->dparams;
     m.norms = s->norms;
+    m.norms_h = s->norms_h;
     m.scratch = s->far;  // written by the far-field kernel after every solve
     return m;
 }

@@ -1,7 +1,6 @@
 // Temporally blocked red-black SOR smoother for the multigrid levels that
-// stream from HBM (edge >= 256; opt-in through PPPM_MG_TB, since the plain
-// half sweeps on groups of 4 cells measured faster inside a whole solve):
-// T half sweeps — T/2 of the
+// stream from HBM (edge >= 256; opt-in through PPPM_MG_TB, since one launch of
+// mg_sweep.cu per red-black sweep is faster): T half sweeps — T/2 of the
 // reference's red-black iterations (MG/Multigrid.cu:202-239, odd cells first,
 // omega = 1.43f) — in one pass over the level, optionally fused with the
 // prolongation by injection that precedes the post-smoothing
@@ -347,7 +346,7 @@ TbVariant make_variant() {
 
 const TbVariant *variants(int *count) {
     // Measured on B200 (256^3, three components, 8 half sweeps): 0.89 ms
-    // (T2 64x16), 0.81 ms (T2 128x32), 0.94 ms for the plain half sweeps;
+    // (T2 64x16), 0.81 ms (T2 128x32), 0.42 ms for the sweep kernel;
     // staging b through the ring beat reading it from global memory, and T = 4
     // lost to its larger halo.
     static const TbVariant v[] = {

@@ -84,11 +84,11 @@ struct TbMaps {
 struct MGPlan {
     int levels = 0;
     Level lv[kMaxLevels];
-    // blocked smoother per level: its variant (-1 = plain half sweeps), tensor
+    // blocked smoother per level: its variant (-1 = the sweep kernel), tensor
     // maps and z-chunk length (levels with edge >= tb_min_edge, x2 allocated),
     // and the device error flag
     int tb_var[kMaxLevels] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1};
-    uint32_t tb_min_edge = 256;  // smaller levels measured faster with the plain half sweeps
+    uint32_t tb_min_edge = 256;  // smaller levels measured faster with one-colour passes
     bool tb_fuse_prolong = false;  // prolongation inside the first post-smoothing pass
     TbMaps tb_maps[kMaxLevels];
     int tb_zchunk[kMaxLevels] = {};
@@ -100,6 +100,7 @@ struct MGPlan {
     const float *vort = nullptr;    // b = -(vort * h2f) from the P2M grid
     const DevParams *P = nullptr;
     double *norms = nullptr;        // [2] device scratch
+    double *norms_h = nullptr;      // [2] pinned host copy, or null
     float *scratch = nullptr;       // [comps][C0] second copy of a level's x while it is smoothed
 };
 
@@ -130,13 +131,31 @@ struct TailArgs {
     const float *b = nullptr;
     double basis[64] = {};
     double lambda[8] = {};
+    // corrected cycle: ghost factors of A, B, C and 1 / diagonal by boundary faces
+    float gA = 0.f, gB = 0.f, gC = 0.f;
+    float4 invA = {}, invB = {};
 };
 int mg_tail_level(const MGPlan &m);
 cudaError_t mg_tail_prepare();
-cudaError_t mg_tail_launch(const MGPlan &m, int level, bool fmg);
+enum TailMode { kTailCycle = 0, kTailFull = 1, kTailCorrected = 2 };
+cudaError_t mg_tail_launch(const MGPlan &m, int level, TailMode mode);
 // One red-black sweep of a level of edge > 32 (mg_sweep.cu).
 cudaError_t mg_sweep_prepare();
-cudaError_t mg_sweep(const float *x, const float *b, const float *xc, float *out, int d, int comps, cudaStream_t st);
+// The corrected cycle's ghost factor of a level (0 on the finest), and its
+// relaxation factor (mg.cu).
+float mg_ghost_factor(int level);
+constexpr float kCorrOmega = 1.25f;
+struct SweepSpec {
+    const float *x = nullptr;   // null: from zero
+    const float *b = nullptr;
+    const float *xc = nullptr;  // coarser level's correction to add first, or null
+    float *out = nullptr;       // or, instead of it:
+    double *psi = nullptr;      // the FP64 iterate the result is added to
+    bool set_psi = false;       // ... or becomes
+    int d = 0, comps = 1;
+    int corrected = -1;         // level of the corrected cycle, -1: the reference's sweep
+};
+cudaError_t mg_sweep(const SweepSpec &sp, cudaStream_t st);
 
 cudaError_t mg_capture_graph(const MGPlan &m, cudaGraphExec_t *exec, unsigned *kernel_nodes);
 
@@ -191,6 +210,7 @@ struct pppm_scene {
     double *psi = nullptr;                // [3][C]
     float *far = nullptr;                 // [3][C]
     double *norms = nullptr;              // [2] residual / rhs squared norms
+    double *norms_h = nullptr;            // their pinned host copy (CONVERGED scenes)
     cudaGraphExec_t mg_graph = nullptr;   // reference-schedule solve, captured once
     unsigned mg_graph_kernels = 0;
     float *mg_x2_pool = nullptr;          // second x copies of the blocked-smoother levels
@@ -322,8 +342,8 @@ cudaError_t radix_sort_pairs(cudaStream_t st, uint32_t N, uint32_t bits, uint32_
                              uint32_t *hist, uint32_t **sorted_key, uint32_t **sorted_idx);
 
 int mg_level_count(uint32_t n);
-// Blocked-smoother choice for new multigrid objects: -1 (the plain half
-// sweeps) unless PPPM_MG_TB in the environment names a variant index, or
+// Blocked-smoother choice for new multigrid objects: -1 (the sweep
+// kernel) unless PPPM_MG_TB in the environment names a variant index, or
 // "auto" (-2: the autotuner picks per level).
 int mg_tb_default_variant();
 bool mg_shape_ok(uint32_t n);
