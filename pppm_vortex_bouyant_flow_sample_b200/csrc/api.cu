@@ -239,7 +239,6 @@ cudaError_t alloc_grid_side(pppm_scene *s) {
     PPPM_CUDA_TRY(dalloc(&s->cell_end, s->C));
     PPPM_CUDA_TRY(dalloc(&s->mflag, s->C));
     PPPM_CUDA_TRY(dalloc(&s->sub_start, 8 * (size_t)s->C));
-    PPPM_CUDA_TRY(dalloc(&s->sub_end, 8 * (size_t)s->C));
     PPPM_CUDA_TRY(cudaMemset(s->mflag, 0, sizeof(uint32_t) * s->C));
     PPPM_CUDA_TRY(dalloc(&s->dparams, 1));
     PPPM_CUDA_TRY(dalloc(&s->norms, 2));
@@ -276,7 +275,6 @@ void destroy_scene(pppm_scene *s) {
     cudaFree(s->cell_end);
     cudaFree(s->mflag);
     cudaFree(s->sub_start);
-    cudaFree(s->sub_end);
     cudaFree(s->dparams);
     cudaFree(s->norms);
     if (s->norms_h) cudaFreeHost(s->norms_h);

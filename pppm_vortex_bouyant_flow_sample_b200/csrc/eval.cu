@@ -472,7 +472,6 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
     const uint32_t *__restrict__ start = ea.start;
     const uint32_t *__restrict__ end = ea.end;
     const uint32_t *__restrict__ sub_start = ea.sub_start;
-    const uint32_t *__restrict__ sub_end = ea.sub_end;
     const float4 *__restrict__ vrec = ea.vrec;
     const float4 *__restrict__ valf = ea.valf;
     const DevParams *__restrict__ P = ea.P;
@@ -659,16 +658,11 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
                         const uint32_t cell = ((uint32_t)ck * n + (uint32_t)cj) * n + (uint32_t)ci;
                         const uint32_t k0 = (cell << 3) | ((uint32_t)(j2 & 1) << 1) | ((uint32_t)(k2 & 1) << 2) |
                                             (uint32_t)(i2 & 1);
-                        uint32_t ps = sub_start[k0], pe = sub_end[k0];
-                        if (both) {
-                            const uint32_t s1 = sub_start[k0 | 1u];
-                            if (s1 != kEmpty) {
-                                if (ps == kEmpty) ps = s1;
-                                pe = sub_end[k0 | 1u];
-                            }
-                        }
+                        const uint32_t cs = start[cell];
+                        const uint32_t ps = sub_start[k0], next = k0 + (both ? 2u : 1u);
+                        const uint32_t pe = (next & 7u) ? sub_start[next] : end[cell];
                         i2 += both ? 2 : 1;
-                        if (ps == kEmpty) continue;
+                        if (cs == kEmpty || ps == pe) continue;
                         stage_run<S, COUNT, FOLD, D>(vrec, valf, ps, pe, cr_lane, ra, rb, pstar, o, blo, bhi,
                                                      dnear, inv_a3_2, cfd, sc.t7, inv4pia3, D == 7 && need_exp2, pk,
                                                      lane, ring, acc2, xf);
@@ -875,7 +869,6 @@ static EvalArgs make_args(pppm_scene *s, const float4 *eval_a, const float4 *eva
     a.start = s->cell_start;
     a.end = s->cell_end;
     a.sub_start = s->sub_start;
-    a.sub_end = s->sub_end;
     a.vrec = s->vrec;
     a.valf = s->valf;
     a.P = s->dparams;

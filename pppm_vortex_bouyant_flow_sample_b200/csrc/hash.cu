@@ -313,15 +313,17 @@ __device__ __forceinline__ uint32_t ngp_cell(float rx, float ry, float rz, doubl
     return ((uint32_t)qz * n + (uint32_t)qy) * n + (uint32_t)qx;
 }
 
-// Cell and sub-cell tables + reorder + relative coordinates + NGP cell, one
-// thread per sorted slot (keys are cell * 8 + octant).  All tables were set
-// to kEmpty beforehand.
+// Cell and octant tables + reorder + relative coordinates + NGP cell, one
+// thread per sorted slot (keys are cell * 8 + octant).  The cell tables were
+// set to kEmpty beforehand; the octant table is valid for non-empty cells only,
+// so that nobody has to clear it (64 B a cell with starts and ends: 1.1 GB at
+// 256^3, most of the 226 us this stage took there).
 __global__ void cells_reorder_kernel(const uint32_t *__restrict__ skey, const uint32_t *__restrict__ sidx,
                                      uint32_t N, const float4 *__restrict__ pos,
                                      const double *__restrict__ alpha, uint32_t capN,
                                      const DevParams *__restrict__ P, uint32_t *__restrict__ start,
                                      uint32_t *__restrict__ end, uint32_t *__restrict__ sub_start,
-                                     uint32_t *__restrict__ sub_end, uint32_t *__restrict__ mflag, uint32_t epoch,
+                                     uint32_t *__restrict__ mflag, uint32_t epoch,
                                      float4 *__restrict__ vrec, float4 *__restrict__ valf) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= N) return;
@@ -333,11 +335,14 @@ __global__ void cells_reorder_kernel(const uint32_t *__restrict__ skey, const ui
         if (s > 0) end[prev >> 3] = s;
     }
     if (s == N - 1) end[key] = N;
-    if (s == 0 || skk != prev) {
-        sub_start[skk] = s;
-        if (s > 0) sub_end[prev] = s;
-    }
-    if (s == N - 1) sub_end[skk] = N;
+    // the octants' first records (an empty octant: where the next begins) of
+    // this cell, written by the records where the octant changes; an octant
+    // ends where the next one begins, the last with the cell
+    const bool head = s == 0 || key != (prev >> 3);
+    const uint32_t oct = skk & 7u;
+    for (uint32_t q = head ? 0u : (prev & 7u) + 1u; q <= oct; q++) sub_start[8 * (size_t)key + q] = s;
+    if (s == N - 1 || (skey[s + 1] >> 3) != key)
+        for (uint32_t q = oct + 1; q < 8; q++) sub_start[8 * (size_t)key + q] = s + 1;
     const uint32_t i = sidx[s];
     const float4 p = pos[i];
     const float rx = (float)((double)p.x - P->origin[0]);
@@ -454,8 +459,6 @@ cudaError_t launch_cells_reorder(pppm_scene *s) {
     const size_t tbytes = sizeof(uint32_t) * (size_t)s->C;
     PPPM_CUDA_TRY(cudaMemsetAsync(s->cell_start, 0xFF, tbytes, s->stream));
     PPPM_CUDA_TRY(cudaMemsetAsync(s->cell_end, 0xFF, tbytes, s->stream));
-    PPPM_CUDA_TRY(cudaMemsetAsync(s->sub_start, 0xFF, 8 * tbytes, s->stream));
-    PPPM_CUDA_TRY(cudaMemsetAsync(s->sub_end, 0xFF, 8 * tbytes, s->stream));
     s->epoch++;
     if (s->epoch == 0) {  // wrapped: restart the mismatch flags
         PPPM_CUDA_TRY(cudaMemsetAsync(s->mflag, 0, tbytes, s->stream));
@@ -464,7 +467,7 @@ cudaError_t launch_cells_reorder(pppm_scene *s) {
     ::pppm::note_launch();
     cells_reorder_kernel<<<blocks_for(s->N, 256), 256, 0, s->stream>>>(
         s->vsorted_key, s->vsorted_idx, s->N, s->vpos, s->valpha, s->capN, s->dparams, s->cell_start,
-        s->cell_end, s->sub_start, s->sub_end, s->mflag, s->epoch, s->vrec, s->valf);
+        s->cell_end, s->sub_start, s->mflag, s->epoch, s->vrec, s->valf);
     return cudaGetLastError();
 }
 

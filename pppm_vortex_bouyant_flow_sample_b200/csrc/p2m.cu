@@ -5,9 +5,8 @@
 // The reference gathers, for every grid cell, over the 5^3 hash cells around
 // it and keeps the particles whose NGP cell is that cell.  Here the vortices
 // are already sorted by hash cell, so a cell's particles are one contiguous
-// run: one warp takes 32 consecutive cells, walks the non-empty runs with
-// coalesced loads, reduces with a fixed xor-butterfly (deterministic, no
-// atomics), and the owning lane writes the cell.  A particle whose FP64 NGP
+// run: a warp walks a cell's run with coalesced loads and reduces with a fixed
+// xor-butterfly (deterministic, no atomics on the sums).  A particle whose FP64 NGP
 // cell differs from its FP32 hash cell (a rounding tie at a cell face) has
 // flagged its NGP cell; only flagged cells also walk their 26 neighbouring
 // runs, which is the exact set the reference's 5^3 window can reach.
@@ -17,7 +16,8 @@ namespace pppm {
 
 namespace {
 
-constexpr int kP2MThreads = 256;
+constexpr int kP2MThreads = 128;
+constexpr int kP2MCells = 128;  // cells of a block
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -28,13 +28,14 @@ __device__ __forceinline__ float warp_sum(float v) {
 __device__ __forceinline__ void run_sum(const float4 *__restrict__ vrec, const float4 *__restrict__ valf,
                                         uint32_t s, uint32_t e, uint32_t cell, int lane, float &ax, float &ay,
                                         float &az) {
-    // unrolled so that a dense cell's loads are in flight together (each
-    // lane's records are still added in order)
+    // unrolled, and the strength loaded whether or not it counts, so that a
+    // dense cell's loads are in flight together (each lane's records are still
+    // added in order)
 #pragma unroll 4
     for (uint32_t p = s + lane; p < e; p += 32) {
-        const float4 r = vrec[p];
-        if (__float_as_uint(r.w) == cell) {
-            const float4 a = valf[p];
+        const uint32_t at = __float_as_uint(vrec[p].w);
+        const float4 a = valf[p];
+        if (at == cell) {
             ax += a.x;
             ay += a.y;
             az += a.z;
@@ -42,39 +43,54 @@ __device__ __forceinline__ void run_sum(const float4 *__restrict__ vrec, const f
     }
 }
 
+// A block takes 128 consecutive cells.  Their runs differ widely (a ring fills
+// a few thousand cells of two million, ten or more in a row, with hundreds of
+// records each), so the block lists its non-empty cells and its warps take
+// them in turn: with a warp for its own 32 cells the longest of them set the
+// time.  1M ring at 128^3: 178 to 127 us; 262,144 points spread over 256^3,
+// bound by the cell bounds and the six grids (134 MB + 400 MB), 152 and 157 us.
 __global__ void __launch_bounds__(kP2MThreads)
 p2m_kernel(const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
            const float4 *__restrict__ vrec, const float4 *__restrict__ valf, const uint32_t *__restrict__ mflag,
            uint32_t epoch, const DevParams *__restrict__ P, uint32_t n, float *__restrict__ vort,
            float *__restrict__ rhs) {
+    __shared__ uint32_t cs[kP2MCells], ce[kP2MCells];
+    __shared__ unsigned char list[kP2MCells], flist[kP2MCells];
+    __shared__ int busy, flagged;
+    __shared__ float sum[3][kP2MCells];
     const uint32_t C = n * n * n;
-    const int lane = threadIdx.x & 31;
-    const uint32_t cell = (blockIdx.x * blockDim.x + threadIdx.x);
-    const uint32_t wbase = cell - lane;
-    if (wbase >= C) return;
-    const bool inb = cell < C;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t base = blockIdx.x * kP2MCells, cell = base + tid;
+    const bool inb = tid < kP2MCells && cell < C;
+    if (tid == 0) busy = flagged = 0;
+    __syncthreads();
     const uint32_t s = inb ? start[cell] : kEmpty;
-    const uint32_t e = inb ? end[cell] : kEmpty;
-    const bool flagged = inb && mflag[cell] == epoch;
-    float ox = 0.f, oy = 0.f, oz = 0.f;  // this lane's cell
-    uint32_t busy = __ballot_sync(0xffffffffu, s != kEmpty);
-    while (busy) {
-        const int b = __ffs(busy) - 1;
-        busy &= busy - 1;
-        const uint32_t cs = __shfl_sync(0xffffffffu, s, b);
-        const uint32_t ce = __shfl_sync(0xffffffffu, e, b);
+    const bool fl = inb && mflag[cell] == epoch;
+    if (tid < kP2MCells) sum[0][tid] = sum[1][tid] = sum[2][tid] = 0.f;
+    if (s != kEmpty) {
+        cs[tid] = s;
+        ce[tid] = end[cell];
+        list[atomicAdd(&busy, 1)] = (unsigned char)tid;  // any order: each cell is summed by itself
+    }
+    if (fl) flist[atomicAdd(&flagged, 1)] = (unsigned char)tid;
+    __syncthreads();
+    for (int q = warp; q < busy; q += kP2MThreads / 32) {
+        const int b = list[q];
         float ax = 0.f, ay = 0.f, az = 0.f;
-        run_sum(vrec, valf, cs, ce, wbase + b, lane, ax, ay, az);
+        run_sum(vrec, valf, cs[b], ce[b], base + b, lane, ax, ay, az);
         ax = warp_sum(ax);
         ay = warp_sum(ay);
         az = warp_sum(az);
-        if (lane == b) { ox = ax; oy = ay; oz = az; }
+        if (lane == 0) {
+            sum[0][b] = ax;
+            sum[1][b] = ay;
+            sum[2][b] = az;
+        }
     }
-    uint32_t fl = __ballot_sync(0xffffffffu, flagged);
-    while (fl) {
-        const int b = __ffs(fl) - 1;
-        fl &= fl - 1;
-        const uint32_t c = wbase + b;
+    __syncthreads();
+    for (int q = warp; q < flagged; q += kP2MThreads / 32) {
+        const int b = flist[q];
+        const uint32_t c = base + b;
         const int ci = (int)(c % n), cj = (int)((c / n) % n), ck = (int)(c / (n * n));
         float ax = 0.f, ay = 0.f, az = 0.f;
         for (int dk = -1; dk <= 1; dk++)
@@ -91,11 +107,16 @@ p2m_kernel(const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
         ax = warp_sum(ax);
         ay = warp_sum(ay);
         az = warp_sum(az);
-        if (lane == b) { ox += ax; oy += ay; oz += az; }
+        if (lane == 0) {
+            sum[0][b] += ax;
+            sum[1][b] += ay;
+            sum[2][b] += az;
+        }
     }
+    __syncthreads();
     if (inb) {
         const float s3 = P->invh3_f, h2 = P->h2f;
-        const float wx = ox * s3, wy = oy * s3, wz = oz * s3;
+        const float wx = sum[0][tid] * s3, wy = sum[1][tid] * s3, wz = sum[2][tid] * s3;
         vort[cell] = wx;
         vort[C + cell] = wy;
         vort[2 * (size_t)C + cell] = wz;
@@ -108,7 +129,7 @@ p2m_kernel(const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
 }  // namespace
 
 cudaError_t launch_p2m(pppm_scene *s) {
-    const unsigned blocks = (s->C + kP2MThreads - 1) / kP2MThreads;
+    const unsigned blocks = (s->C + kP2MCells - 1) / kP2MCells;
     ::pppm::note_launch();
     p2m_kernel<<<blocks, kP2MThreads, 0, s->stream>>>(s->cell_start, s->cell_end, s->vrec, s->valf, s->mflag,
                                                       s->epoch, s->dparams, s->n, s->vort, s->lv[0].b);

@@ -197,7 +197,7 @@ struct pppm_scene {
     float4 *vrec = nullptr;               // sorted {rel, ngp}
     float4 *valf = nullptr;               // sorted {alpha, 0}
     uint32_t *cell_start = nullptr, *cell_end = nullptr, *mflag = nullptr;
-    uint32_t *sub_start = nullptr, *sub_end = nullptr;   // [8 n^3] runs of (cell, octant)
+    uint32_t *sub_start = nullptr;        // [8 n^3] first record of (cell, octant), non-empty cells only
     uint32_t epoch = 0;
 
     // radix-sort histogram scratch
@@ -289,7 +289,7 @@ struct EvalArgs {
     uint32_t M;
     const float4 *eval_a, *eval_b;
     const float *far;
-    const uint32_t *start, *end, *sub_start, *sub_end;
+    const uint32_t *start, *end, *sub_start;
     const float4 *vrec, *valf;
     const DevParams *P;
     int n, K;

@@ -74,7 +74,7 @@ uint64_t scene_footprint(uint32_t n, uint32_t N) {
     uint64_t levels = 0, d = n;
     while (d * d * d > 512) { levels += d * d * d; d /= 2; }
     levels += d * d * d;
-    const uint64_t grid = C * (12 /*vort*/ + 24 /*psi*/ + 12 /*far*/ + 12 /*start,end,flag*/ + 64 /*sub tables*/) +
+    const uint64_t grid = C * (12 /*vort*/ + 24 /*psi*/ + 12 /*far*/ + 12 /*start,end,flag*/ + 32 /*octant table*/) +
                           levels * 24 /*mg x,b*/;
     const uint64_t part = (uint64_t)N * (16 + 24 + 32 /*sort*/ + 32 /*records*/ + 16 /*rk2*/ + 16 /*ref order*/ +
                                          32 /*eval sort*/ + 32 /*staging*/ + 16 + 24 + 24 /*server arrays*/);

@@ -1,4 +1,4 @@
-"""The multigrid's level kernels at the edges where they change: the launch
+"""The grid kernels at the edges where they change.  The multigrid: the launch
 that holds the levels of edge <= 32 (csrc/mg_tail.cu: slabs of 4 planes of a
 level of edge 17 to 32, the level of edge 9 to 16 and the coarsest one), and
 the fused red-black sweep of the larger levels (csrc/mg_sweep.cu: whole rows,
@@ -67,3 +67,25 @@ def test_corrected_cycles_reach_the_tolerance(pb, oracle, n, tol):
     got = np.linalg.norm(r) / np.linalg.norm(b)
     assert got <= tol
     assert abs(rel - got) <= 1e-6 * got + 1e-14
+
+
+@pytest.mark.parametrize("K", [-1, 0, 1, 2, 4])
+@pytest.mark.parametrize("n", [10, 12, 20])
+def test_far_field_grid(pb, oracle, n, K):
+    """The far-field grid of the four-cell kernel (edges that are multiples of
+    4: rows of 3 and 5 groups, windows beyond both ends) and of the one-cell
+    kernel (10): FP32 sums of at most 728 terms beside an FP64 curl, so 1e-5."""
+    import torch
+    rng = np.random.default_rng(5)
+    N = 900
+    pos = np.zeros((N, 4), np.float32)
+    pos[:, :3] = rng.uniform(0.0, 1.0, (N, 3))
+    al = rng.normal(size=(N, 3))
+    box = dict(fixed_origin=(0.0, 0.0, 0.0), fixed_length=1.0)
+    scene = pb.Scene(n, K=K, cap_vort=N, cap_eval=N, domain="fixed", **box)
+    scene.set_vortices(torch.from_numpy(pos).cuda(), torch.from_numpy(np.ascontiguousarray(al.T)).cuda())
+    scene.build_far_field()
+    far = scene.grid(pb.GRID_FAR).cpu().numpy()
+    scene.close()
+    d = oracle.pppm(oracle.params(n, K=K, domain_mode=1, **box), pos, al, pos[:4], None, 0, dump=True)[1]
+    assert rel_l2(far, d["far_u"]) <= 1e-5
