@@ -5,8 +5,9 @@
 //  * cell keys bit-exact with PH/particle_hash_kernel.cu:32-70;
 //  * a stable LSD radix sort of (key, index) replacing thrust::sort_by_key
 //    (PH/SpaceHashFunctional.cu:97-102): 8-bit digits, per pass an upsweep
-//    histogram, one scan, and a downsweep whose ranks are stable (warp
-//    __match_any_sync, warps and item rounds in index order);
+//    histogram, one scan, and a downsweep whose ranks are stable (warps and
+//    item rounds in index order); up to 8,192 pairs are sorted by one block
+//    in one launch;
 //  * cell start/end tables (PH/particle_hash_kernel.cu:74-126) fused with the
 //    gather of positions and strengths into sorted order
 //    (PH/particle_hash_kernel.cu:128-158), which also rounds positions to the
@@ -69,7 +70,23 @@ __device__ float float_below(double c) {
 
 __global__ void params_kernel(const float *__restrict__ partial, int nblocks, pppm_params prm,
                               DevParams *__restrict__ P) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    // one warp reduces the blocks' partial boxes (a single thread took 22 us
+    // over 296 blocks, a load at a time), its first lane forms the parameters
+    float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+    for (int b = threadIdx.x; b < nblocks; b += 32)
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            lo[a] = fminf(lo[a], partial[a * nblocks + b]);
+            hi[a] = fmaxf(hi[a], partial[(3 + a) * nblocks + b]);
+        }
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
+            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+        }
+    if (threadIdx.x != 0) return;
     double origin[3], L;
     if (prm.domain_mode == PPPM_DOMAIN_FIXED) {
         origin[0] = prm.fixed_origin[0];
@@ -79,13 +96,8 @@ __global__ void params_kernel(const float *__restrict__ partial, int nblocks, pp
     }
     double mn[3], mx[3];
     for (int a = 0; a < 3; a++) {
-        float lo = partial[a * nblocks], hi = partial[(3 + a) * nblocks];
-        for (int b = 1; b < nblocks; b++) {
-            lo = fminf(lo, partial[a * nblocks + b]);
-            hi = fmaxf(hi, partial[(3 + a) * nblocks + b]);
-        }
-        mn[a] = lo;
-        mx[a] = hi;
+        mn[a] = lo[a];
+        mx[a] = hi[a];
     }
     if (prm.domain_mode != PPPM_DOMAIN_FIXED) {
         // HFS/BiotSavartSolverImp.cpp:399-406
@@ -203,10 +215,26 @@ radix_upsweep_kernel(const uint32_t *__restrict__ keys, uint32_t N, int shift, u
     cnt[threadIdx.x] = 0;
     __syncthreads();
     const uint32_t base = blockIdx.x * kRsTile;
-#pragma unroll 4
-    for (int j = 0; j < kRsItems; j++) {
-        uint32_t i = base + j * kRsThreads + threadIdx.x;
-        if (i < N) atomicAdd(&cnt[(keys[i] >> shift) & 255u], 1u);
+    uint4 k[kRsItems / 4];
+#pragma unroll
+    for (int j = 0; j < kRsItems / 4; j++) {
+        const uint32_t i = base + 4 * (j * kRsThreads + threadIdx.x);
+        if (i + 3 < N) {
+            k[j] = *reinterpret_cast<const uint4 *>(keys + i);
+        } else {
+            k[j].x = i < N ? keys[i] : 0u;
+            k[j].y = i + 1 < N ? keys[i + 1] : 0u;
+            k[j].z = i + 2 < N ? keys[i + 2] : 0u;
+            k[j].w = 0u;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kRsItems / 4; j++) {
+        const uint32_t i = base + 4 * (j * kRsThreads + threadIdx.x);
+        if (i < N) atomicAdd(&cnt[(k[j].x >> shift) & 255u], 1u);
+        if (i + 1 < N) atomicAdd(&cnt[(k[j].y >> shift) & 255u], 1u);
+        if (i + 2 < N) atomicAdd(&cnt[(k[j].z >> shift) & 255u], 1u);
+        if (i + 3 < N) atomicAdd(&cnt[(k[j].w >> shift) & 255u], 1u);
     }
     __syncthreads();
     hist[threadIdx.x * gridDim.x + blockIdx.x] = cnt[threadIdx.x];
@@ -253,55 +281,176 @@ radix_rowscan_kernel(uint32_t *__restrict__ hist, uint32_t nb, uint32_t *__restr
     if (threadIdx.x == 0) totals[blockIdx.x] = run;
 }
 
-// Stable scatter of one 8-bit digit.  Item order inside a tile is
-// (round j, warp, lane) = index order, so ranks preserve input order.
+// Ranks of one 8-bit digit for the keys of a block's warps: each warp counts
+// its own contiguous keys, kItems rounds of 32 lanes in index order, in its own
+// 256 counters, so a round needs no block barrier.  The equal digits of a round
+// are found bit by bit with ballots, and their first lane moves the counter.
+// k[]: the keys, all ones past the end; rank[]: a key's place among the warp's
+// equal digits.
+template <int kItems>
+__device__ __forceinline__ void warp_ranks(const uint32_t (&k)[kItems], int shift, uint32_t *__restrict__ cnt,
+                                           uint32_t (&rank)[kItems], int lane) {
+    const uint32_t lt_mask = (1u << lane) - 1u;
+#pragma unroll
+    for (int j = 0; j < kItems; j++) {
+        const uint32_t d = (k[j] >> shift) & 255u;
+        uint32_t peers = 0xffffffffu;
+#pragma unroll
+        for (int b = 0; b < 8; b++) {
+            const uint32_t set = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+            peers &= ((d >> b) & 1u) ? set : ~set;
+        }
+        const uint32_t before = cnt[d];
+        __syncwarp();
+        if ((peers & lt_mask) == 0u) cnt[d] = before + __popc(peers);
+        __syncwarp();
+        rank[j] = before + __popc(peers & lt_mask);
+    }
+}
+
+// Stable scatter of one 8-bit digit: a warp takes kRsItems * 32 consecutive
+// keys of the tile, the tile is put in digit order in shared memory, and each
+// digit's run is then written by consecutive threads.  With a block barrier for
+// each round of 256 keys and the keys written where they fell, a pass over 1M
+// keys took 14 us; so it takes 9 (16 MB: 2.5 us at the copy rate; the ranks'
+// serial rounds are the rest).  The counts before it, with 128-bit loads and
+// a warp's own counters: 6.4 to 3.0 us.
 __global__ void __launch_bounds__(kRsThreads)
 radix_downsweep_kernel(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
                        uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, uint32_t N, int shift,
                        const uint32_t *__restrict__ hist, const uint32_t *__restrict__ totals) {
-    __shared__ uint32_t goff[256];
-    __shared__ uint32_t running[256];
-    __shared__ uint32_t wcnt[kRsWarps][256];
+    __shared__ uint32_t cnt[kRsWarps][256];
+    __shared__ uint32_t place[256];  // first output slot of a digit less its first place in the tile
     __shared__ uint32_t warp_tot[kRsWarps];
+    __shared__ uint32_t sk[kRsTile], sv[kRsTile];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t base = blockIdx.x * kRsTile, first = base + (uint32_t)warp * (kRsItems * 32) + lane;
+    for (int q = 0; q < kRsWarps; q++) cnt[q][tid] = 0;
+    uint32_t k[kRsItems], v[kRsItems], rank[kRsItems];
+#pragma unroll
+    for (int j = 0; j < kRsItems; j++) {
+        const uint32_t i = first + 32u * j;
+        k[j] = i < N ? kin[i] : 0xFFFFFFFFu;
+        v[j] = i < N ? vin[i] : 0u;
+    }
     uint32_t all;
     const uint32_t digit_base = block_excl_scan256(totals[tid], warp_tot, all);
-    goff[tid] = digit_base + hist[tid * gridDim.x + blockIdx.x];
-    running[tid] = 0;
-    const uint32_t lt_mask = (1u << lane) - 1u;
-    const uint32_t base = blockIdx.x * kRsTile;
-    for (int j = 0; j < kRsItems; j++) {
-        for (int q = 0; q < kRsWarps; q++) wcnt[q][tid] = 0;
-        __syncthreads();
-        const uint32_t i = base + j * kRsThreads + tid;
-        const bool valid = i < N;
-        uint32_t k = 0, d = 256u + lane;  // invalid lanes form singleton groups
-        if (valid) {
-            k = kin[i];
-            d = (k >> shift) & 255u;
-        }
-        const uint32_t peers = __match_any_sync(0xffffffffu, d);
-        const uint32_t rank = __popc(peers & lt_mask);
-        if (valid && rank == 0) wcnt[warp][d] = __popc(peers);
-        __syncthreads();
-        {
-            uint32_t acc = running[tid];
+    warp_ranks<kRsItems>(k, shift, cnt[warp], rank, lane);
+    __syncthreads();
+    uint32_t mine = 0;  // this thread's digit: its count in the tile, the warps' offsets in it
 #pragma unroll
-            for (int q = 0; q < kRsWarps; q++) {
-                uint32_t c = wcnt[q][tid];
-                wcnt[q][tid] = acc;
-                acc += c;
-            }
-            running[tid] = acc;
-        }
-        __syncthreads();
-        if (valid) {
-            const uint32_t p = goff[d] + wcnt[warp][d] + rank;
-            kout[p] = k;
-            vout[p] = vin[i];
-        }
-        __syncthreads();
+    for (int q = 0; q < kRsWarps; q++) {
+        const uint32_t c = cnt[q][tid];
+        cnt[q][tid] = mine;
+        mine += c;
     }
+    const uint32_t start = block_excl_scan256(mine, warp_tot, all);
+#pragma unroll
+    for (int q = 0; q < kRsWarps; q++) cnt[q][tid] += start;
+    place[tid] = digit_base + hist[tid * gridDim.x + blockIdx.x] - start;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kRsItems; j++) {
+        // keys past the end rank behind every other (all ones, last in order)
+        const uint32_t at = cnt[warp][(k[j] >> shift) & 255u] + rank[j];
+        sk[at] = k[j];
+        sv[at] = v[j];
+    }
+    __syncthreads();
+    const uint32_t live = min((uint32_t)kRsTile, N - base);
+    for (uint32_t at = tid; at < live; at += kRsThreads) {
+        const uint32_t key = sk[at], to = place[(key >> shift) & 255u] + at;
+        kout[to] = key;
+        vout[to] = sv[at];
+    }
+}
+
+// The whole sort in one block for up to kSmallMax pairs: the keys and values
+// stay in registers between passes and change places through shared memory.
+// Three launches a pass, each as long as a launch takes, otherwise make most
+// of a small scene's sorts: 11 + 3.5 + 2 us a pass for 2,000 keys, 80 us for a
+// scene's five passes, against 15 us for its two sorts here.  One block ranks
+// 16,384 keys in 63 us a sort where the tiles take 36, hence the limit.
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr uint32_t kSmallMax = 8192;
+
+template <int kItems>
+__global__ void __launch_bounds__(kSmallThreads)
+radix_small_kernel(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin, uint32_t *__restrict__ kout,
+                   uint32_t *__restrict__ vout, uint32_t N, uint32_t bits) {
+    extern __shared__ uint32_t small_smem[];
+    uint32_t *cnt = small_smem;                                  // [kSmallWarps][256]
+    uint32_t *sk = cnt + kSmallWarps * 256, *sv = sk + kItems * kSmallThreads;
+    __shared__ uint32_t tot[8];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t first = (uint32_t)warp * (kItems * 32) + lane;
+    uint32_t k[kItems], v[kItems], rank[kItems];
+#pragma unroll
+    for (int j = 0; j < kItems; j++) {
+        const uint32_t i = first + 32u * j;
+        k[j] = i < N ? kin[i] : 0xFFFFFFFFu;
+        v[j] = i < N ? vin[i] : 0u;
+    }
+    for (uint32_t shift = 0; shift < bits; shift += 8) {
+        for (int q = tid; q < kSmallWarps * 256; q += kSmallThreads) cnt[q] = 0;
+        __syncthreads();
+        warp_ranks<kItems>(k, (int)shift, cnt + warp * 256, rank, lane);
+        __syncthreads();
+        uint32_t mine = 0;
+        if (tid < 256) {
+#pragma unroll 8
+            for (int q = 0; q < kSmallWarps; q++) {
+                const uint32_t c = cnt[q * 256 + tid];
+                cnt[q * 256 + tid] = mine;
+                mine += c;
+            }
+        }
+        uint32_t x = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (tid < 256 && lane == 31) tot[warp] = x;
+        __syncthreads();
+        if (tid < 256) {
+            uint32_t start = x - mine;
+            for (int q = 0; q < warp; q++) start += tot[q];
+#pragma unroll 8
+            for (int q = 0; q < kSmallWarps; q++) cnt[q * 256 + tid] += start;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kItems; j++) {
+            const uint32_t at = cnt[warp * 256 + ((k[j] >> shift) & 255u)] + rank[j];
+            sk[at] = k[j];
+            sv[at] = v[j];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kItems; j++) {
+            k[j] = sk[first + 32u * j];
+            v[j] = sv[first + 32u * j];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kItems; j++) {
+        const uint32_t i = first + 32u * j;
+        if (i < N) {
+            kout[i] = k[j];
+            vout[i] = v[j];
+        }
+    }
+}
+
+template <int kItems>
+cudaError_t launch_small_sort(cudaStream_t st, uint32_t N, uint32_t bits, uint32_t *key[2], uint32_t *idx[2], int to) {
+    const size_t smem = sizeof(uint32_t) * (kSmallWarps * 256 + 2 * kItems * kSmallThreads);
+    PPPM_CUDA_TRY(cudaFuncSetAttribute(radix_small_kernel<kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ::pppm::note_launch();
+    radix_small_kernel<kItems><<<1, kSmallThreads, smem, st>>>(key[0], idx[0], key[to], idx[to], N, bits);
+    return cudaGetLastError();
 }
 
 __device__ __forceinline__ uint32_t ngp_cell(float rx, float ry, float rz, double invh, uint32_t n) {
@@ -419,6 +568,16 @@ cudaError_t radix_sort_pairs(cudaStream_t st, uint32_t N, uint32_t bits, uint32_
                                     uint32_t **sorted_idx) {
     const uint32_t nb = (N + kRsTile - 1) / kRsTile;
     int cur = 0;
+    if (N <= kSmallMax) {
+        // the result lands where the passes of the larger sort leave it
+        cur = (int)((bits + 7) / 8) & 1;
+        PPPM_CUDA_TRY(N <= kSmallMax / 4   ? launch_small_sort<2>(st, N, bits, key, idx, cur)
+                      : N <= kSmallMax / 2 ? launch_small_sort<4>(st, N, bits, key, idx, cur)
+                                           : launch_small_sort<8>(st, N, bits, key, idx, cur));
+        *sorted_key = key[cur];
+        *sorted_idx = idx[cur];
+        return cudaSuccess;
+    }
     for (uint32_t shift = 0; shift < bits; shift += 8) {
         ::pppm::note_launch();
         radix_upsweep_kernel<<<nb, kRsThreads, 0, st>>>(key[cur], N, (int)shift, hist);

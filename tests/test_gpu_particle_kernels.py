@@ -1,5 +1,6 @@
-"""The particle kernels at the sizes where their paths change: the deposit of
-cells with very different numbers of vortices."""
+"""The particle kernels at the sizes where their paths change: the sort in one
+block and in tiles, and the deposit of cells with very different numbers of
+vortices."""
 import numpy as np
 import pytest
 
@@ -29,6 +30,27 @@ def _points(rng, N, lo=0.0, hi=1.0):
     p = np.zeros((N, 4), np.float32)
     p[:, :3] = rng.uniform(lo, hi, (N, 3))
     return p
+
+
+@pytest.mark.parametrize("N", [1, 33, 2048, 2049, 4096, 4097, 8191, 8192, 8193, 12289])
+@pytest.mark.parametrize("n", [8, 48])
+def test_sort_is_stable_at_every_size(pb, n, N):
+    """Keys ascending, equal keys in index order, every index once: the block
+    sort (to 8,192 pairs, 2, 4 or 8 a thread), the tiles (4,096) and their
+    remainders, two and three digits of key."""
+    rng = np.random.default_rng(N)
+    pm = pb.ParticleManager()
+    pm.initSpatialHash(N, n, n, n)
+    pm.setSpatialHashGrid(n, 1.0 / n, (0.0, 0.0, 0.0), N)
+    pos = _points(rng, N)
+    pm.doSpatialHash(_dev(pos), N)
+    key, idx = pm.getHashTable().numpy(), pm.getIndexTable().numpy()
+    pm.endSpatialHash()
+    c = np.floor(pos[:, :3] / np.float32(1.0 / n)).astype(np.int64) % n
+    want = (c[:, 2] * n + c[:, 1]) * n + c[:, 0]
+    order = np.argsort(want, kind="stable")
+    assert np.array_equal(idx, order)
+    assert np.array_equal(key, want[order])
 
 
 def test_deposit_of_uneven_cells(pb, oracle):
