@@ -49,6 +49,7 @@ struct pppm_potential {
     size_t hist_cap = 0;
     uint32_t *sidx = nullptr;
     uint32_t *start = nullptr, *end = nullptr;
+    unsigned char *tie = nullptr;  // grid cells that also take particles of neighbouring hash cells
     float4 *srec = nullptr;   // sorted {rel.x, rel.y, rel.z, 0}
     double *smass = nullptr;  // sorted masses
     // grids (FP64)
@@ -97,34 +98,57 @@ __global__ void pot_bbox_kernel(const float4 *__restrict__ pos, uint32_t N, floa
     }
 }
 
+// Sorted records, and the flag of every grid cell that a particle of another
+// hash cell lies nearest to (a rounding tie at a cell face).
 __global__ void pot_records_kernel(const float4 *__restrict__ pos, const double *__restrict__ mass,
-                                   const uint32_t *__restrict__ sidx, uint32_t N, double ox, double oy, double oz,
-                                   float4 *__restrict__ srec, double *__restrict__ smass) {
+                                   const uint32_t *__restrict__ skey, const uint32_t *__restrict__ sidx, uint32_t N,
+                                   double ox, double oy, double oz, double invh, int d, float4 *__restrict__ srec,
+                                   double *__restrict__ smass, unsigned char *__restrict__ tie) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= N) return;
     const uint32_t i = sidx[s];
     const float4 p = pos[i];
-    srec[s] = make_float4((float)((double)p.x - ox), (float)((double)p.y - oy), (float)((double)p.z - oz), 0.f);
+    const float4 r = make_float4((float)((double)p.x - ox), (float)((double)p.y - oy), (float)((double)p.z - oz), 0.f);
+    srec[s] = r;
     smass[s] = mass[i];
+    // cells whose half-open box [c - 1/2, c + 1/2) about the centre may hold
+    // the particle, by the deposit's own expression; only ties have others
+    // than the hash cell
+    const double q[3] = {(double)r.x * invh, (double)r.y * invh, (double)r.z * invh};
+    const double f[3] = {floor(q[0]), floor(q[1]), floor(q[2])};
+    const uint32_t key = skey[s];
+    const int hi = (int)(key % d), hj = (int)((key / d) % d), hk = (int)(key / ((uint32_t)d * d));
+    const double near = 1e-6;  // far beyond the rounding of q - (c + 1/2)
+    const bool tied = f[0] != hi || f[1] != hj || f[2] != hk || q[0] - f[0] < near || q[0] - f[0] > 1.0 - near ||
+                      q[1] - f[1] < near || q[1] - f[1] > 1.0 - near || q[2] - f[2] < near || q[2] - f[2] > 1.0 - near;
+    if (!tied) return;
+    for (int c = 0; c < 27; c++) {
+        const int ii = hi + c % 3 - 1, jj = hj + (c / 3) % 3 - 1, kk = hk + c / 9 - 1;
+        if (ii >= 0 && jj >= 0 && kk >= 0 && ii < d && jj < d && kk < d) tie[((uint32_t)kk * d + jj) * d + ii] = 1;
+    }
 }
 
 // ParticleToMesh_kernel (HFS/GPU_kernel.cu:218-294): a particle adds m to the
 // cell whose centre lies within half a cell on every axis (NGP, in FP64 on
 // the float relative coordinate).  That cell is the particle's hash cell or a
-// neighbour, so the 3^3 hash cells around the grid cell hold every candidate.
+// neighbour, so the 3^3 hash cells around the grid cell hold every candidate,
+// and unless a tie is flagged its own hash cell does (128^3: 100 us with the
+// 27 runs of every cell, 23 us so).
 // Then rhs = -(h_f^2) rho (ComputeRHS, h_f^2 rounded to float).
 __global__ void pot_p2m_kernel(const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
-                               const float4 *__restrict__ srec, const double *__restrict__ smass, int d,
-                               double invh, double h2, double *__restrict__ rho, double *__restrict__ rhs) {
+                               const float4 *__restrict__ srec, const double *__restrict__ smass,
+                               const unsigned char *__restrict__ tie, int d, double invh, double h2,
+                               double *__restrict__ rho, double *__restrict__ rhs) {
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= (uint32_t)d * d * d) return;
     const int i = (int)(c % d), j = (int)((c / d) % d), k = (int)(c / ((uint32_t)d * d));
     const double gx = (double)(float)((double)i + 0.5), gy = (double)(float)((double)j + 0.5),
                  gz = (double)(float)((double)k + 0.5);
     double sum = 0.0;
-    for (int kk = max(k - 1, 0); kk <= min(k + 1, d - 1); kk++)
-        for (int jj = max(j - 1, 0); jj <= min(j + 1, d - 1); jj++)
-            for (int ii = max(i - 1, 0); ii <= min(i + 1, d - 1); ii++) {
+    const int w = tie[c] ? 1 : 0;
+    for (int kk = max(k - w, 0); kk <= min(k + w, d - 1); kk++)
+        for (int jj = max(j - w, 0); jj <= min(j + w, d - 1); jj++)
+            for (int ii = max(i - w, 0); ii <= min(i + w, d - 1); ii++) {
                 const uint32_t r = ((uint32_t)kk * d + jj) * d + ii;
                 const uint32_t s0 = start[r];
                 if (s0 == kEmpty) continue;
@@ -170,11 +194,16 @@ __global__ void pot_mono_partial_kernel(const float4 *__restrict__ pos, const do
     }
 }
 
+// One warp, a strided share of the blocks' partial sums a lane (a single thread
+// over all of them took 44 us).
 __global__ void pot_mono_final_kernel(const double *__restrict__ part, int nb, double *__restrict__ mono) {
-    if (threadIdx.x != 0) return;
     double a[5] = {0, 0, 0, 0, 0};
-    for (int q = 0; q < 5; q++)
-        for (int b = 0; b < nb; b++) a[q] += part[q * nb + b];
+#pragma unroll
+    for (int q = 0; q < 5; q++) {
+        for (int b = threadIdx.x; b < nb; b += 32) a[q] += part[q * nb + b];
+        for (int o = 16; o > 0; o >>= 1) a[q] += __shfl_xor_sync(0xffffffffu, a[q], o);
+    }
+    if (threadIdx.x != 0) return;
     mono[0] = a[2] / a[0];
     mono[1] = a[3] / a[0];
     mono[2] = a[4] / a[0];
@@ -220,15 +249,11 @@ __device__ __forceinline__ void periodic_grad(const double *__restrict__ f, int 
     g[2] = 1.0 * (b - fr) * 0.5 * invh;
 }
 
-// Gradient buffer: far = grad(phi) - sum_{c' != 0} D[c'] m(c + c')
-// - grad(0.250580605913965 rho h^2), every gradient periodic central
-// differences; D is the central-difference gradient of 1/(4 pi r) between
-// cell centres, built per block in shared memory.
-__global__ void pot_far_gradient_kernel(const double *__restrict__ phi, const double *__restrict__ rho, int d, int K,
-                                        double h, double *__restrict__ far) {
-    extern __shared__ double table[];  // [3][(2K+1)^3]
+// D of the gradient buffer below, [3][(2K+1)^3]: the central-difference
+// gradient of 1/(4 pi r) between cell centres.
+__device__ void gradient_table(double *__restrict__ table, double h, int K, int tid, int threads) {
     const int W = 2 * K + 1, T = W * W * W;
-    for (int e = threadIdx.x; e < T; e += blockDim.x) {
+    for (int e = tid; e < T; e += threads) {
         const int ii = e % W - K, jj = (e / W) % W - K, kk = e / (W * W) - K;
         double tx = 0, ty = 0, tz = 0;
         if (!(ii == 0 && jj == 0 && kk == 0)) {
@@ -246,6 +271,17 @@ __global__ void pot_far_gradient_kernel(const double *__restrict__ phi, const do
         table[T + e] = ty;
         table[2 * T + e] = tz;
     }
+}
+
+// Gradient buffer: far = grad(phi) - sum_{c' != 0} D[c'] m(c + c')
+// - grad(0.250580605913965 rho h^2), every gradient periodic central
+// differences; D is the central-difference gradient of 1/(4 pi r) between
+// cell centres, built per block in shared memory.
+__global__ void pot_far_gradient_kernel(const double *__restrict__ phi, const double *__restrict__ rho, int d, int K,
+                                        double h, double *__restrict__ far) {
+    extern __shared__ double table[];  // [3][(2K+1)^3]
+    const int W = 2 * K + 1, T = W * W * W;
+    gradient_table(table, h, K, (int)threadIdx.x, (int)blockDim.x);
     __syncthreads();
     const uint32_t C = (uint32_t)d * d * d;
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -277,6 +313,80 @@ __global__ void pot_far_gradient_kernel(const double *__restrict__ phi, const do
     far[c] = (g[0] - fm[0]) - gd[0];
     far[C + c] = (g[1] - fm[1]) - gd[1];
     far[2 * (size_t)C + c] = (g[2] - fm[2]) - gd[2];
+}
+
+// The same with a thread per pair of consecutive cells of a row (even edge):
+// each of the (2K+1)^2 neighbour rows is read once for both with 128-bit loads,
+// and each table entry once, the terms of a cell in the one-cell kernel's
+// order (cells beyond the grid add a zero).  K = 1 at 128^3 on B200: 124 to
+// 59 us (its 40 bytes a cell take 13 us at the copy rate; the rest is FP64
+// arithmetic, 156 multiply-adds a cell).
+template <int K>
+__global__ void __launch_bounds__(128)
+pot_far_gradient2_kernel(const double *__restrict__ phi, const double *__restrict__ rho, int d, double h,
+                         double *__restrict__ far) {
+    constexpr int W = 2 * K + 1, T = W * W * W;
+    constexpr int R = (K + 1) / 2 * 2;  // values loaded either side of the pair
+    __shared__ double table[3 * T];
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+    gradient_table(table, h, K, tid, (int)(blockDim.x * blockDim.y));
+    __syncthreads();
+    const uint32_t C = (uint32_t)d * d * d, dd = (uint32_t)d * d;
+    const int i0 = 2 * (int)(blockIdx.x * blockDim.x + threadIdx.x), j = (int)(blockIdx.y * blockDim.y + threadIdx.y);
+    const int k = (int)blockIdx.z;
+    if (i0 >= d || j >= d) return;
+    const double invh = 1.0 / h;
+    const double v = h * h * h;
+    double fm[2][3] = {};
+#pragma unroll 1
+    for (int kk = k - K; kk <= k + K; kk++) {
+        if (kk < 0 || kk >= d) continue;
+#pragma unroll 1
+        for (int jj = j - K; jj <= j + K; jj++) {
+            if (jj < 0 || jj >= d) continue;
+            const double *row = rho + ((uint32_t)kk * d + jj) * d + i0;
+            double m[2 + 2 * R];
+#pragma unroll
+            for (int q = -R; q < 2 + R; q += 2) {
+                const bool in = i0 + q >= 0 && i0 + q < d;
+                const double2 a = in ? *reinterpret_cast<const double2 *>(row + q) : make_double2(0.0, 0.0);
+                m[q + R] = kG * a.x * v;
+                m[q + R + 1] = kG * a.y * v;
+            }
+            const int e0 = ((kk - k + K) * W + (jj - j + K)) * W + K;
+#pragma unroll
+            for (int di = -K; di <= K; di++) {
+                const double tx = table[e0 + di], ty = table[T + e0 + di], tz = table[2 * T + e0 + di];
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    fm[e][0] += tx * m[e + di + R];
+                    fm[e][1] += ty * m[e + di + R];
+                    fm[e][2] += tz * m[e + di + R];
+                }
+            }
+        }
+    }
+    const double dg = 0.250580605913965 * h * h * kG;
+    double out[3][2];
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        const int i = i0 + e;
+        const uint32_t c = ((uint32_t)k * d + j) * d + i;
+        double g[3];
+        periodic_grad(phi, d, c, i, j, k, invh, g);
+        // diagonal term: its periodic gradient from the six neighbours' densities
+        const double rl = rho[c - i + (i + d - 1) % d], rr = rho[c - i + (i + 1) % d];
+        const double rd = rho[c - j * d + ((j + d - 1) % d) * d], rt = rho[c - j * d + ((j + 1) % d) * d];
+        const double rf = rho[c - k * dd + ((k + d - 1) % d) * dd], rb = rho[c - k * dd + ((k + 1) % d) * dd];
+        const double gd[3] = {1.0 * (dg * rr - dg * rl) * 0.5 * invh, 1.0 * (dg * rt - dg * rd) * 0.5 * invh,
+                              1.0 * (dg * rb - dg * rf) * 0.5 * invh};
+#pragma unroll
+        for (int q = 0; q < 3; q++) out[q][e] = (g[q] - fm[e][q]) - gd[q];
+    }
+    const uint32_t c = ((uint32_t)k * d + j) * d + i0;
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+        *reinterpret_cast<double2 *>(far + q * (size_t)C + c) = make_double2(out[q][0], out[q][1]);
 }
 
 __global__ void pot_gradient_only_kernel(const double *__restrict__ phi, int d, double h, double *__restrict__ far) {
@@ -557,6 +667,7 @@ extern "C" pppm_status pppm_potential_create(uint32_t n, int K, uint32_t cap_mas
     const size_t C = P->C;
     if (e == cudaSuccess) e = grow(&P->start, C);
     if (e == cudaSuccess) e = grow(&P->end, C);
+    if (e == cudaSuccess) e = grow(&P->tie, C);
     if (e == cudaSuccess) e = grow(&P->density, C);
     if (e == cudaSuccess) e = grow(&P->rhs, C);
     if (e == cudaSuccess) e = grow(&P->phi, C);
@@ -586,7 +697,7 @@ extern "C" pppm_status pppm_potential_destroy(pppm_potential *P) {
     for (int q = 0; q < 2; q++) {
         cudaFree(P->key[q]); cudaFree(P->idx[q]); cudaFree(P->ekey[q]); cudaFree(P->eidx[q]);
     }
-    cudaFree(P->hist); cudaFree(P->start); cudaFree(P->end); cudaFree(P->srec); cudaFree(P->smass);
+    cudaFree(P->hist); cudaFree(P->start); cudaFree(P->end); cudaFree(P->tie); cudaFree(P->srec); cudaFree(P->smass);
     cudaFree(P->density); cudaFree(P->rhs); cudaFree(P->phi); cudaFree(P->far); cudaFree(P->mono);
     cudaFree(P->mono_part); cudaFree(P->bbox);
     if (P->host_bbox) cudaFreeHost(P->host_bbox);
@@ -653,14 +764,16 @@ extern "C" pppm_status pppm_potential_build(pppm_potential *P, int scalar) {
     const double invh = 1.0 / P->cell_h;
     if (e == cudaSuccess) {
         note_launch();
-        pot_records_kernel<<<(N + 255) / 256, 256, 0, st>>>(P->mpos, P->mass, P->sidx, N, P->origin[0], P->origin[1],
-                                                             P->origin[2], P->srec, P->smass);
-        e = cudaGetLastError();
+        e = cudaMemsetAsync(P->tie, 0, C, st);
+        pot_records_kernel<<<(N + 255) / 256, 256, 0, st>>>(P->mpos, P->mass, skey, P->sidx, N, P->origin[0],
+                                                             P->origin[1], P->origin[2], invh, (int)n, P->srec,
+                                                             P->smass, P->tie);
+        if (e == cudaSuccess) e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
         note_launch();
-        pot_p2m_kernel<<<(C + 255) / 256, 256, 0, st>>>(P->start, P->end, P->srec, P->smass, (int)n, invh,
-                                                        (double)(P->h_f * P->h_f), P->density, P->rhs);
+        pot_p2m_kernel<<<(C + 255) / 256, 256, 0, st>>>(P->start, P->end, P->srec, P->smass, P->tie, (int)n,
+                                                        invh, (double)(P->h_f * P->h_f), P->density, P->rhs);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
@@ -682,7 +795,15 @@ extern "C" pppm_status pppm_potential_build(pppm_potential *P, int scalar) {
     const int K = P->K;
     if (!scalar) {
         note_launch();
-        if (K >= 0) {
+        if (K >= 0 && n % 2 == 0) {
+            const int bx = (int)std::min(32u, n / 2);
+            const dim3 block(bx, 128 / bx), grid((n / 2 + block.x - 1) / block.x, (n + block.y - 1) / block.y, n);
+            auto *f = K == 0 ? pot_far_gradient2_kernel<0>
+                             : (K == 1 ? pot_far_gradient2_kernel<1>
+                                       : (K == 2 ? pot_far_gradient2_kernel<2>
+                                                 : (K == 3 ? pot_far_gradient2_kernel<3> : pot_far_gradient2_kernel<4>)));
+            f<<<grid, block, 0, st>>>(P->phi, P->density, (int)n, P->cell_h, P->far);
+        } else if (K >= 0) {
             const int W = 2 * K + 1;
             const size_t smem = sizeof(double) * 3 * (size_t)W * W * W;
             pot_far_gradient_kernel<<<(C + 127) / 128, 128, smem, st>>>(P->phi, P->density, (int)n, K, P->cell_h,
