@@ -4,9 +4,9 @@
 // :2262-2485 BiotSavartPPCorrScaleMN_kernel, PH/particle_hash_kernel.cu:
 // 160-188 removeReorder).
 //
-// Evaluation points are visited in hash order (same grid as the vortices), so
-// the threads of a warp walk the same neighbour cells and read the same
-// vortex records.  Per point:
+// Evaluation points are visited along a Hilbert curve, so that the threads of a
+// warp walk the same neighbour cells and read the same vortex records.  Per
+// point:
 //   * relative position rounded to float from the FP64 difference with the
 //     domain origin, NGP cell floor(rel * invh) in FP64 (reference rounding);
 //   * far field: hat weights 1 - |cell centre - rel/h| on the 8 surrounding
@@ -41,54 +41,65 @@ namespace pppm {
 namespace {
 
 constexpr int kEvalThreads = 128;
-// Resident blocks per SM the evaluation kernels are compiled for: 9 (56
-// registers, a few bytes of spill outside the pair loop) measured 12.85 ms on
-// the 1M-ring headline against 13.05 ms with 8 (64 registers) and 13.77 ms
-// with 10 (48 registers).
-constexpr int kEvalBlocksPerSM = 9;
+// 72 registers.  The pair loop is bound by issue slots and the latency of its
+// special functions: 1M points on 128^3 with a of a cell (exp form) take 12.2 ms
+// with 7 blocks, 12.3 with 6 (80 registers), 12.5 with 8 (64); 2M segment ends on
+// 256^3 (polynomial) 1.30 ms with 7, 1.39 with 6, 1.43 with 8.
+constexpr int kEvalBlocksPerSM = 7;
 
 __device__ __forceinline__ float3 rel_pos(float4 p, const DevParams *__restrict__ P) {
     return make_float3((float)((double)p.x - P->origin[0]), (float)((double)p.y - P->origin[1]),
                        (float)((double)p.z - P->origin[2]));
 }
 
-// Evaluation order: NGP cell, then the Gray rank of the point's octant inside
-// the cell, then (fine = 1) the Gray rank of its quarter-cell inside the
-// octant (points outside the grid last).  A warp of consecutive points then
-// covers about a quarter of a cell, so the union of its lanes' near-field
-// boxes, over which it walks, exceeds each lane's own box by little and few
-// staged candidates fail the lane's box test.  The order is internal: results
-// return in caller order.
+// Evaluation order: along a Hilbert curve through the quarter cells of the
+// grid (half cells where four times the edge needs more than 10 bits), points
+// outside at the nearest one.  32 consecutive points then lie close together
+// on all three axes whatever the density, so that the union of their
+// near-field boxes, over which a warp walks, exceeds each point's own box by
+// little.  Rows of cells, however ordered inside, string the points of a
+// sparse scene out along x: 32 of them spanned 20 cells of a 256^3 grid with
+// 1.5 vortices a cell.  The order is internal: results return in caller order.
+// The curve's index by Skilling's transform (AIP Conf. Proc. 707, 381, 2004):
+// undo the rotations from the top bit down, then take the Gray code.
+__device__ __forceinline__ uint32_t hilbert_index(uint32_t x, uint32_t y, uint32_t z, int bits) {
+    uint32_t v[3] = {x, y, z};
+    for (int b = bits - 1; b > 0; b--) {
+        const uint32_t q = 1u << b, low = q - 1u;
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            if (v[a] & q) {
+                v[0] ^= low;
+            } else {
+                const uint32_t t = (v[0] ^ v[a]) & low;
+                v[0] ^= t;
+                v[a] ^= t;
+            }
+        }
+    }
+    v[1] ^= v[0];
+    v[2] ^= v[1];
+    uint32_t t = 0;
+    for (int b = bits - 1; b > 0; b--)
+        if (v[2] & (1u << b)) t ^= (1u << b) - 1u;
+    uint32_t key = 0;
+    for (int b = bits - 1; b >= 0; b--)
+#pragma unroll
+        for (int a = 0; a < 3; a++) key = (key << 1) | (((v[a] ^ t) >> b) & 1u);
+    return key;
+}
+
 __global__ void eval_keys_kernel(const float4 *__restrict__ eval_a, uint32_t M, const DevParams *__restrict__ P,
-                                 int fine, uint32_t *__restrict__ key, uint32_t *__restrict__ idx) {
+                                 int per_cell, int bits, uint32_t *__restrict__ key, uint32_t *__restrict__ idx) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= M) return;
     const float3 r = rel_pos(eval_a[t], P);
-    const double invh = P->invh;
-    const uint32_t n = P->n;
-    const double qx = (double)r.x * invh, qy = (double)r.y * invh, qz = (double)r.z * invh;
-    const double fx = floor(qx), fy = floor(qy), fz = floor(qz);
-    const double dn = (double)n;
-    const int sh = fine ? 6 : 3;
-    uint32_t k = (n * n * n) << sh;
-    if (fx >= 0.0 && fx < dn && fy >= 0.0 && fy < dn && fz >= 0.0 && fz < dn) {
-        // quarter-cell coordinates 0..3 per axis (clamped against rounding)
-        const uint32_t ux = min(3u, (uint32_t)(4.0 * (qx - fx))), uy = min(3u, (uint32_t)(4.0 * (qy - fy))),
-                       uz = min(3u, (uint32_t)(4.0 * (qz - fz)));
-        const uint32_t oct = (ux >> 1) | ((uy >> 1) << 1) | ((uz >> 1) << 2);
-        // groups in Gray-code order (0,1,3,2,6,7,5,4): neighbouring groups differ
-        // along one axis, so a warp spanning two groups widens its walk on one
-        // axis only
-        const uint32_t rank = (0x54672310u >> (4 * oct)) & 7u;
-        const uint32_t cell = ((uint32_t)fz * n + (uint32_t)fy) * n + (uint32_t)fx;
-        if (fine) {
-            const uint32_t sub = (ux & 1u) | ((uy & 1u) << 1) | ((uz & 1u) << 2);
-            k = (cell << 6) | (rank << 3) | ((0x54672310u >> (4 * sub)) & 7u);
-        } else {
-            k = (cell << 3) | rank;
-        }
-    }
-    key[t] = k;
+    const double scale = P->invh * (double)per_cell, top = (double)(P->n * (uint32_t)per_cell - 1u);
+    // (a coordinate that is not a number goes to 0)
+    const uint32_t ux = (uint32_t)fmin(fmax((double)r.x * scale, 0.0), top),
+                   uy = (uint32_t)fmin(fmax((double)r.y * scale, 0.0), top),
+                   uz = (uint32_t)fmin(fmax((double)r.z * scale, 0.0), top);
+    key[t] = hilbert_index(ux, uy, uz, bits);
     idx[t] = t;
 }
 
@@ -156,38 +167,51 @@ __device__ __forceinline__ void cell_pairs(const float4 *__restrict__ vrec, cons
         pair_term<SEG, COUNT, false>(vrec[p], valf[p], lane_ok, ra, rb, cr, inv_a3, cf, inv4pia3, need_exp, acc);
 }
 
-// Packed accumulators of the warp-uniform walk (.x half: even records of a
-// staged chunk, .y half: odd ones).  The near-field sum
-//   sum_p c_p alpha_p x (ra - r_p)
+// The near-field sum of a target,
+//   sum_p c_p alpha_p x (ra - r_p),
 // is kept as  A x (ra - o) - B  with  A = sum_p c_p alpha_p  and
-// B = sum_p c_p alpha_p x (r_p - o), o a point of the warp's neighbourhood
-// (lane 0's position): the per-source moment alpha_p x (r_p - o) is formed
-// once when the record is staged, so a pair costs 6 multiply-adds for the
-// accumulation instead of 9 for a cross product per pair.  With o within a few
-// cells of both points, the two terms are of the size of the result (no
-// cancellation beyond a few ulp).
-struct PairAcc2 {
-    float2 ax = {0.f, 0.f}, ay = {0.f, 0.f}, az = {0.f, 0.f};
+// B = sum_p c_p alpha_p x (r_p - o), o the middle of the warp's targets: the
+// per-source moment alpha_p x (r_p - o) is formed once when the record is
+// staged, so a pair costs 6 multiply-adds for the accumulation instead of 9 for
+// a cross product per pair.  With o within a few cells of both points, the two
+// terms are of the size of the result (no cancellation beyond a few ulp).
+struct PairSums {
+    float2 ax = {0.f, 0.f}, ay = {0.f, 0.f}, az = {0.f, 0.f};  // .x half: even records, .y half: odd ones
     float2 bx = {0.f, 0.f}, by = {0.f, 0.f}, bz = {0.f, 0.f};
     unsigned long long n = 0;
 };
 
-// Per-warp ring of staged vortex records: 64 records as 32 record pairs, so
-// that one Blackwell f32x2 instruction (FADD2 / FMUL2 / FFMA2) works on two
-// records: slot p holds records 2p (.x, .z halves) and 2p+1 (.y, .w halves).
+// Ring of a warp: 64 records as 32 record pairs, so that one Blackwell f32x2
+// instruction (FADD2 / FMUL2 / FFMA2) works on two records and a lane on its
+// own target: slot p holds records 2p (.x, .z halves) and 2p+1 (.y, .w halves).
 // Planes: A {-x, -y}, B {-z, alpha_x}, C {alpha_y, alpha_z}, D {m_x, m_y},
-// E {m_z} with m = alpha x (r - o).  Records kept from successive runs are
-// appended (record i at slot (i / 2) mod 32) and evaluated 32 at a time, so
-// the pair loop runs whole blocks of 16 slots whatever the lengths of the
-// runs; only the last block of a walk is partial.
-constexpr int kPackSlots = 32;
-constexpr int kPackPlanes = 5;
+// E {m_z, index} with m = alpha x (r - o).
+// The sums are a contraction, coefficients (targets x sources) times source
+// columns (alpha, m), but as one it is slower: with the coefficients in the
+// layout of m16n8k8, split into two TF32 parts to keep FP32's digits, 1M points
+// on 128^3 with a of a cell took 15.0 ms against 12.2 ms here, and 262,144
+// segments' ends 2.35 ms against 1.78 ms.  The product frees 12 of the 53 issue slots of
+// two pairs, the split and the layout take 8 back, and 4 targets x 8 sources of
+// coefficients a lane leave too few registers to hide the special functions.
+constexpr int kRingSlots = 32;
+constexpr int kRingPlanes = 5;
 constexpr uint32_t kBlockRecs = 32;  // records per block of the pair loop
+// What a warp's walk needs per chunk of records but not per pair, kept out of
+// the registers of the pair block.
+struct WarpBox {
+    float4 lo, hi;   // the targets' boxes' union; lo.w: margin of the near test
+    float4 mid;      // origin of the moments
+    int4 cells, size;  // first cell x, half-cells y, z and x; cells x, half-cells y, z and last half-cell x
+};
+struct WarpMem {
+    float4 ring[kRingPlanes * kRingSlots];
+    WarpBox box;
+};
 
 struct Ring {
     uint32_t fill = 0;  // records staged so far
     uint32_t head = 0;  // records evaluated so far (a multiple of kBlockRecs)
-    bool near = false;  // a waiting record may lie within a / 4 of a lane (exp form)
+    bool near = false;  // a waiting record may lie within a / 4 of a target (exp form)
 };
 
 // max(|a|, |b|, |c|) in one instruction: the three-input max.abs of PTX ISA 8.8
@@ -238,63 +262,112 @@ struct ExpForm {
 // branch on nearly every step.
 constexpr float kExpSmallT = 1.0f / 64.0f;
 
-// WIDX: the record's index into the sorted vortices goes to E's spare half
-// (the index test of segment evaluation).
-template <bool WIDX = false>
-__device__ __forceinline__ void stage_record(float *__restrict__ pk, int slot, int half, float4 r, float4 a,
-                                             float3 o, uint32_t ridx = 0xFFFFFFFFu) {
-    float *A = pk + 4 * (0 * kPackSlots + slot), *B = pk + 4 * (1 * kPackSlots + slot);
-    float *Cc = pk + 4 * (2 * kPackSlots + slot), *D = pk + 4 * (3 * kPackSlots + slot);
-    float *E = pk + 4 * (4 * kPackSlots + slot);
-    const float sx = r.x - o.x, sy = r.y - o.y, sz = r.z - o.z;
-    A[half] = -r.x; A[2 + half] = -r.y;
-    B[half] = -r.z; B[2 + half] = a.x;
-    Cc[half] = a.y; Cc[2 + half] = a.z;
-    D[half] = fmaf(a.y, sz, -(a.z * sy)); D[2 + half] = fmaf(a.z, sx, -(a.x * sz));
-    E[half] = fmaf(a.x, sy, -(a.y * sx));
-    if (WIDX) E[2 + half] = __uint_as_float(ridx);
+// The exp form of two pairs at (dx, dy, dz): c * 4 pi = (1 - e^-t) / r^3 with
+// t = r^3 / a^3: r^-1 from rsqrt, e^-t from ex2 (two special-function ops).
+// r^2 gets 1e-30 in its chain, so that rsqrt stays finite at r = 0.  Where some
+// lane has t < tsmall (1 - e^-t cancels, or r = 0) the degree-5 polynomial
+// phi(t) / a^3 replaces it; CHECK: whether it is looked for.  The trigger
+// r^3 < r3small is a superset of t < tsmall, and a pair outside its box may
+// trigger it (its coefficient is dropped either way).
+template <bool CHECK>
+__device__ __forceinline__ float2 exp_coeff(float2 dx, float2 dy, float2 dz, const float2 *cf, const ExpForm &xf) {
+    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, make_float2(1e-30f, 1e-30f))));
+    const float2 rs = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
+    const float2 r3 = __fmul2_rn(r2, __fmul2_rn(r2, rs));
+    const float2 ri3 = __fmul2_rn(__fmul2_rn(rs, rs), rs);
+    const float2 ex = __fmul2_rn(r3, xf.nl2a3);
+    const float2 e = make_float2(ex2_approx(ex.x), ex2_approx(ex.y));
+    float2 c = __ffma2_rn(make_float2(-e.x, -e.y), ri3, ri3);
+    if (CHECK && __any_sync(0xffffffffu, fminf(r3.x, r3.y) < xf.r3small)) {
+        const float2 t = __fmul2_rn(r3, xf.inv_a3);
+        float2 p = __ffma2_rn(cf[5], t, cf[4]);
+#pragma unroll
+        for (int q = 3; q >= 0; q--) p = __ffma2_rn(p, t, cf[q]);
+        p = __fmul2_rn(p, xf.inv_a3);
+        c.x = t.x < xf.tsmall ? p.x : c.x;
+        c.y = t.y < xf.tsmall ? p.y : c.y;
+    }
+    return c;
 }
 
-// The pair loop over np slots of the ring from slot s0 (FULL: one whole block
-// of 16 slots, unrolled into straight-line code with constant offsets): every
-// lane takes the records two at a time from shared memory (broadcast reads)
-// and evaluates both pairs with packed f32x2 arithmetic.  cr_lane is the box
-// half-width, or -1 for an inactive lane.  The r = 0 exclusion needs no test:
-// the pair's (ra - r_p) is zero.  SEG: the other-end test, 1 by position
-// (|rb - r_p|^2 < 1e-24), 2 by record index (the one vortex at rb, pstar, found
-// beforehand), 0 none.  phi is the
-// degree-DEG polynomial cf (DEG 4: the scene never leaves [0, 0.25]; DEG 7:
-// valid on [0, 2], the exp form above tbig when need_exp; DEG 0: the exp form,
-// the polynomial only for small t, looked for only when CHECK).  FOLD: the
-// coefficients carry the powers of 1/a^3, so the polynomial takes r^3
-// directly and tbig is in r^3 too.
-template <int SEG, bool COUNT, bool FOLD, int DEG, bool FULL, bool CHECK>
-__device__ __forceinline__ void pair_slots(const float4 *__restrict__ pk4, uint32_t s0, uint32_t np, float cr_lane,
-                                           const float3 ra, const float3 rb, uint32_t pstar, float2 inv_a3,
-                                           const float2 *cf, float tbig, float inv4pia3, bool need_exp,
-                                           PairAcc2 &acc, const ExpForm &xf) {
+// phi of two pairs at (dx, dy, dz): the degree-DEG polynomial cf (DEG 4: the
+// scene never leaves [0, 0.25]; DEG 7: valid on [0, 2], the exp form above tbig
+// when need_exp), or (DEG 0) the exp form.  FOLD: the coefficients carry the
+// powers of 1/a^3, so the polynomial takes r^3 directly and tbig is in r^3 too.
+template <bool FOLD, int DEG, bool CHECK>
+__device__ __forceinline__ float2 phi_coeff(float2 dx, float2 dy, float2 dz, bool ok0, bool ok1, float2 inv_a3,
+                                            const float2 *cf, float tbig, float inv4pia3, bool need_exp,
+                                            const ExpForm &xf) {
+    float2 c;
+    if constexpr (DEG == 0) {
+        c = exp_coeff<CHECK>(dx, dy, dz, cf, xf);
+    } else {
+        const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+        const float2 r3 = __fmul2_rn(r2, make_float2(sqrt_approx(r2.x), sqrt_approx(r2.y)));
+        const float2 t3 = FOLD ? r3 : __fmul2_rn(r3, inv_a3);
+        c = __ffma2_rn(cf[DEG], t3, cf[DEG - 1]);
+#pragma unroll
+        for (int q = DEG - 2; q >= 0; q--) c = __ffma2_rn(c, t3, cf[q]);
+        if (DEG > 4 && need_exp) {
+            const bool big0 = ok0 && t3.x >= tbig, big1 = ok1 && t3.y >= tbig;
+            if (__any_sync(0xffffffffu, big0 || big1)) {
+                const float v0 = FOLD ? t3.x * inv_a3.x : t3.x, v1 = FOLD ? t3.y * inv_a3.y : t3.y;
+                const float e0 = __fdividef(1.0f - __expf(-v0), fmaxf(v0, 1.0f)) * inv4pia3;
+                const float e1 = __fdividef(1.0f - __expf(-v1), fmaxf(v1, 1.0f)) * inv4pia3;
+                c.x = big0 ? e0 : c.x;
+                c.y = big1 ? e1 : c.y;
+            }
+        }
+    }
+    return c;
+}
+
+// Puts a record (position r, strength a, moments about o) at place e of a ring.
+__device__ __forceinline__ void stage_record(WarpMem &W, uint32_t e, float4 r, float4 a, float3 o, uint32_t ridx) {
+    const uint32_t slot = (e >> 1) & (kRingSlots - 1), half = e & 1u;
+    float *A = reinterpret_cast<float *>(&W.ring[slot]) + half;
+    constexpr int kPlane = 4 * kRingSlots;
+    const float sx = r.x - o.x, sy = r.y - o.y, sz = r.z - o.z;
+    A[0] = -r.x;
+    A[2] = -r.y;
+    A[kPlane] = -r.z;
+    A[kPlane + 2] = a.x;
+    A[2 * kPlane] = a.y;
+    A[2 * kPlane + 2] = a.z;
+    A[3 * kPlane] = fmaf(a.y, sz, -(a.z * sy));
+    A[3 * kPlane + 2] = fmaf(a.z, sx, -(a.x * sz));
+    A[4 * kPlane] = fmaf(a.x, sy, -(a.y * sx));
+    A[4 * kPlane + 2] = __uint_as_float(ridx);
+}
+
+// np slots of the ring from slot s0 (FULL: one whole block of 16 slots,
+// unrolled into straight-line code with constant offsets): every lane takes
+// the records two at a time (broadcast reads).  cr_lane: the half-width of the
+// box, or -1 for a lane without a point.  OTHER: the other-end test of segments,
+// 1 by position (|rb - r_p|^2 < 1e-24), 2 by record index (the one vortex at rb,
+// pstar, found beforehand), 0 none.  The r = 0 exclusion needs no test: the
+// pair's ra - r_p is zero.
+template <int OTHER, bool COUNT, bool FOLD, int DEG, bool FULL, bool CHECK>
+__device__ __forceinline__ void pair_block(const WarpMem &W, uint32_t s0, uint32_t np, float cr_lane,
+                                             const float3 ra, const float3 rb, uint32_t pstar, float2 inv_a3,
+                                             const float2 *cf, float tbig, float inv4pia3, bool need_exp,
+                                             const ExpForm &xf, PairSums &acc) {
     const float2 tx = make_float2(ra.x, ra.x), ty = make_float2(ra.y, ra.y), tz = make_float2(ra.z, ra.z);
     const uint32_t cnt = FULL ? kBlockRecs / 2 : np;
 #pragma unroll (FULL ? kBlockRecs / 2 : 2)
     for (uint32_t i = 0; i < cnt; i++) {
-        const uint32_t p = s0 + i;
-        const float4 A = pk4[0 * kPackSlots + p], B = pk4[1 * kPackSlots + p], Cc = pk4[2 * kPackSlots + p];
-        const float4 D = pk4[3 * kPackSlots + p], E = pk4[4 * kPackSlots + p];
+        const float4 *pk = &W.ring[s0 + i];
+        const float4 A = pk[0], B = pk[kRingSlots], Cc = pk[2 * kRingSlots];
+        const float4 D = pk[3 * kRingSlots], E = pk[4 * kRingSlots];
         const float2 nx = make_float2(A.x, A.y), ny = make_float2(A.z, A.w), nz = make_float2(B.x, B.y);
         const float2 dx = __fadd2_rn(tx, nx), dy = __fadd2_rn(ty, ny), dz = __fadd2_rn(tz, nz);
-        const float m0 = max3_abs(dx.x, dy.x, dz.x);
-        const float m1 = max3_abs(dx.y, dy.y, dz.y);
-        // (the exp form adds 1e-30 to r^2 in the chain, so that rsqrt stays
-        // finite at r = 0; that pair takes the polynomial below)
-        const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, make_float2(DEG == 0 ? 1e-30f : 0.f,
-                                                                                    DEG == 0 ? 1e-30f : 0.f))));
-        bool ok0 = m0 <= cr_lane, ok1 = m1 <= cr_lane;
+        bool ok0 = max3_abs(dx.x, dy.x, dz.x) <= cr_lane, ok1 = max3_abs(dx.y, dy.y, dz.y) <= cr_lane;
         if (COUNT) acc.n += (ok0 ? 1ull : 0ull) + (ok1 ? 1ull : 0ull);
-        if (SEG == 2) {
+        if (OTHER == 2) {
             ok0 = ok0 && __float_as_uint(E.z) != pstar;
             ok1 = ok1 && __float_as_uint(E.w) != pstar;
         }
-        if (SEG == 1) {
+        if (OTHER == 1) {
             const float2 ex = __fadd2_rn(make_float2(rb.x, rb.x), nx);
             const float2 ey = __fadd2_rn(make_float2(rb.y, rb.y), ny);
             const float2 ez = __fadd2_rn(make_float2(rb.z, rb.z), nz);
@@ -302,51 +375,11 @@ __device__ __forceinline__ void pair_slots(const float4 *__restrict__ pk4, uint3
             ok0 = ok0 && !(e2.x < 1e-24f);
             ok1 = ok1 && !(e2.y < 1e-24f);
         }
-        float2 c;
-        if constexpr (DEG == 0) {
-            // exp form, c * 4 pi = (1 - e^-t) / r^3 with t = r^3 / a^3: r^-1
-            // from rsqrt, e^-t from ex2 (two special-function ops); where
-            // some lane has t < tsmall (1 - e^-t cancels, or r = 0) the
-            // degree-5 polynomial phi(t) / a^3 replaces it
-            const float2 rs = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
-            const float2 r3 = __fmul2_rn(r2, __fmul2_rn(r2, rs));
-            const float2 ri3 = __fmul2_rn(__fmul2_rn(rs, rs), rs);
-            const float2 ex = __fmul2_rn(r3, xf.nl2a3);
-            const float2 e = make_float2(ex2_approx(ex.x), ex2_approx(ex.y));
-            c = __ffma2_rn(make_float2(-e.x, -e.y), ri3, ri3);
-            // the trigger r^3 < r3small is a superset of t < tsmall, and
-            // a lane outside its box may trigger it (its coefficient is
-            // dropped below either way)
-            if (CHECK && __any_sync(0xffffffffu, fminf(r3.x, r3.y) < xf.r3small)) {
-                const float2 t = __fmul2_rn(r3, xf.inv_a3);
-                float2 p = __ffma2_rn(cf[5], t, cf[4]);
-#pragma unroll
-                for (int q = 3; q >= 0; q--) p = __ffma2_rn(p, t, cf[q]);
-                p = __fmul2_rn(p, xf.inv_a3);
-                c.x = t.x < xf.tsmall ? p.x : c.x;
-                c.y = t.y < xf.tsmall ? p.y : c.y;
-            }
-        } else {
-            const float2 r3 = __fmul2_rn(r2, make_float2(sqrt_approx(r2.x), sqrt_approx(r2.y)));
-            const float2 t = FOLD ? r3 : __fmul2_rn(r3, inv_a3);
-            c = __ffma2_rn(cf[DEG], t, cf[DEG - 1]);
-#pragma unroll
-            for (int q = DEG - 2; q >= 0; q--) c = __ffma2_rn(c, t, cf[q]);
-            if (DEG > 4 && need_exp) {
-                const bool big0 = ok0 && t.x >= tbig, big1 = ok1 && t.y >= tbig;
-                if (__any_sync(0xffffffffu, big0 || big1)) {
-                    const float v0 = FOLD ? t.x * inv_a3.x : t.x, v1 = FOLD ? t.y * inv_a3.y : t.y;
-                    const float e0 = __fdividef(1.0f - __expf(-v0), fmaxf(v0, 1.0f)) * inv4pia3;
-                    const float e1 = __fdividef(1.0f - __expf(-v1), fmaxf(v1, 1.0f)) * inv4pia3;
-                    c.x = big0 ? e0 : c.x;
-                    c.y = big1 ? e1 : c.y;
-                }
-            }
-        }
-        // the exp form's c is finite for every pair of an active lane (r = 0
-        // lies inside the box and takes the polynomial), so the box mask can
-        // multiply it; the polynomials can overflow on the padding record
-        const float2 coeff = (DEG == 0 && SEG != 1 && !COUNT)
+        const float2 c = phi_coeff<FOLD, DEG, CHECK>(dx, dy, dz, ok0, ok1, inv_a3, cf, tbig, inv4pia3, need_exp, xf);
+        // the exp form's c is finite for every pair of a lane with a point (r = 0
+        // takes the polynomial), so the box mask can multiply it; the polynomials
+        // can overflow on the padding record
+        const float2 coeff = (DEG == 0 && OTHER != 1 && !COUNT)
                                  ? __fmul2_rn(c, make_float2(ok0 ? 1.0f : 0.0f, ok1 ? 1.0f : 0.0f))
                                  : make_float2(ok0 ? c.x : 0.0f, ok1 ? c.y : 0.0f);
         acc.ax = __ffma2_rn(coeff, make_float2(B.z, B.w), acc.ax);
@@ -358,90 +391,14 @@ __device__ __forceinline__ void pair_slots(const float4 *__restrict__ pk4, uint3
     }
 }
 
-// Appends one run of vortex records [ps, pe) to the ring, 32 at a time (one
-// coalesced load per stream).  Records outside the warp's box [blo, bhi]
-// (every lane's box, widened beyond float rounding) cannot pass any lane's
-// test and are dropped.  Whenever 32 records wait, the warp evaluates them.
-// The ring never overwrites a record still waiting: before a chunk fewer than
-// 32 wait, a chunk adds at most 32, and the ring holds 64.
-// Exp form: a record farther than dnear inside the warp's box [blo, bhi] on
-// some axis is more than a / 4 (with a margin) from every lane's point, so no
-// pair with it needs the small-t polynomial; a block of 32 records with no
-// other record skips the warp's test for it.  The records still waiting after
-// a block all come from the chunk just staged (fewer than 32 waited before
-// it), so that chunk's flag carries over.
-template <int SEG, bool COUNT, bool FOLD, int DEG>
-__device__ __forceinline__ void stage_run(const float4 *__restrict__ vrec, const float4 *__restrict__ valf,
-                                          uint32_t ps, uint32_t pe, float cr_lane, const float3 ra,
-                                          const float3 rb, uint32_t pstar, float3 o, const float3 blo,
-                                          const float3 bhi,
-                                          float dnear, float2 inv_a3, const float2 *cf, float tbig,
-                                          float inv4pia3, bool need_exp, float4 *__restrict__ pk4, int lane,
-                                          Ring &ring, PairAcc2 &acc, const ExpForm &xf) {
-    float *pk = reinterpret_cast<float *>(pk4);
-    for (uint32_t base = ps; base < pe; base += 32) {
-        const uint32_t cnt = min(32u, pe - base);
-        // the strength is loaded with the position (one latency per chunk,
-        // not two), also for records the box test then drops
-        bool keep = false;
-        float4 r = make_float4(0.f, 0.f, 0.f, 0.f), al = r;
-        if ((uint32_t)lane < cnt) {
-            r = vrec[base + lane];
-            al = valf[base + lane];
-            keep = r.x >= blo.x && r.x <= bhi.x && r.y >= blo.y && r.y <= bhi.y && r.z >= blo.z && r.z <= bhi.z;
-        }
-        const unsigned kept = __ballot_sync(0xffffffffu, keep);
-        if (kept == 0u) continue;
-        bool near_chunk = true;
-        if (DEG == 0) {
-            const bool nr = keep && r.x >= blo.x + dnear && r.x <= bhi.x - dnear && r.y >= blo.y + dnear &&
-                            r.y <= bhi.y - dnear && r.z >= blo.z + dnear && r.z <= bhi.z - dnear;
-            near_chunk = __any_sync(0xffffffffu, nr);
-        }
-        if (keep) {
-            const uint32_t dst = ring.fill + (uint32_t)__popc(kept & ((1u << lane) - 1u));
-            stage_record<SEG == 2>(pk, (int)((dst >> 1) & (kPackSlots - 1)), (int)(dst & 1u), r, al, o, base + lane);
-        }
-        ring.fill += (uint32_t)__popc(kept);
-        ring.near = ring.near || near_chunk;
-        if (ring.fill - ring.head >= kBlockRecs) {
-            __syncwarp();
-            const uint32_t s0 = (ring.head >> 1) & (kPackSlots - 1);
-            if (DEG != 0 || ring.near)
-                pair_slots<SEG, COUNT, FOLD, DEG, true, true>(pk4, s0, 0, cr_lane, ra, rb, pstar, inv_a3, cf, tbig,
-                                                              inv4pia3, need_exp, acc, xf);
-            else
-                pair_slots<SEG, COUNT, FOLD, DEG, true, false>(pk4, s0, 0, cr_lane, ra, rb, pstar, inv_a3, cf,
-                                                               tbig, inv4pia3, need_exp, acc, xf);
-            ring.head += kBlockRecs;
-            ring.near = near_chunk && ring.fill != ring.head;
-            __syncwarp();  // the next records may take the slots just read
-        }
-    }
-}
-
-// Evaluates the records left in the ring after the walk (fewer than 32); an
-// odd count is padded with a record at (-1e18, -1e18, -1e18) and zero
-// strength, outside every box.
-template <int SEG, bool COUNT, bool FOLD, int DEG>
-__device__ __forceinline__ void finish_ring(float cr_lane, const float3 ra, const float3 rb, uint32_t pstar,
-                                            float2 inv_a3,
-                                            const float2 *cf, float tbig, float inv4pia3, bool need_exp,
-                                            float4 *__restrict__ pk4, int lane, const Ring &ring, PairAcc2 &acc,
-                                            const ExpForm &xf) {
-    const uint32_t rem = ring.fill - ring.head;
-    if (rem == 0) return;
-    if (lane == 0 && (rem & 1u))
-        stage_record<SEG == 2>(reinterpret_cast<float *>(pk4), (int)((ring.fill >> 1) & (kPackSlots - 1)), 1,
-                     make_float4(-1e18f, -1e18f, -1e18f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f),
-                     make_float3(0.f, 0.f, 0.f));
-    __syncwarp();
-    pair_slots<SEG, COUNT, FOLD, DEG, false, true>(pk4, (ring.head >> 1) & (kPackSlots - 1), (rem + 1) >> 1, cr_lane,
-                                                   ra, rb, pstar, inv_a3, cf, tbig, inv4pia3, need_exp, acc, xf);
-    __syncwarp();
-}
-
-constexpr int kUniformMaxSub = 1000;  // warp-uniform walk up to 10^3 half-cells
+// Warp-uniform walk up to this many half-cells (a sparse scene's 32 targets
+// span several cells); beyond, scattered targets walk their own boxes.
+constexpr int kUniformMaxSub = 4096;
+// ... and while the targets span no more than this many cells: the moments
+// about their middle lose digits to the distance from there, and with a few
+// vortices a cell most of the pairs of a block would lie outside the targets'
+// boxes.
+constexpr double kMaxSpread = 2.5;
 
 // SEG: is_segment == 1 with a distinct other-end array (with eval_b == eval_a
 // the other-end test is the r = 0 test itself, so SEG is off).
@@ -459,11 +416,12 @@ struct SmoothSeries {
     float t7;      // 2 in the packed polynomials' variable: where the exp form takes over
 };
 
-// One block of evaluation points (kEvalThreads consecutive points in the
-// evaluation order) of one scene.
-template <bool SEG, bool COUNT, bool FOLD>
+// One block of evaluation points of one scene: kEvalThreads consecutive points
+// in the evaluation order, or (SPLIT) 32 points, whose walk the block's four
+// warps share.
+template <bool SEG, bool COUNT, bool FOLD, bool SPLIT>
 __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalArgs &ea, uint32_t block,
-                                            float4 *__restrict__ stage) {
+                                            WarpMem *__restrict__ stage) {
     const uint32_t *__restrict__ eidx = ea.eidx;
     const uint32_t M = ea.M;
     const float4 *__restrict__ eval_a = ea.eval_a;
@@ -482,43 +440,25 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
     float *__restrict__ uf = ea.uf;
     unsigned long long *__restrict__ pair_count = ea.pair_count;
     const int lane = threadIdx.x & 31;
-    float4 *pk = stage + (threadIdx.x >> 5) * (kPackPlanes * kPackSlots);
-    const uint32_t s = block * blockDim.x + threadIdx.x;
+    const int warp = threadIdx.x >> 5;
+    WarpMem &W = stage[warp];
+    const uint32_t s = SPLIT ? block * 32 + lane : block * blockDim.x + threadIdx.x;
     const bool act = s < M;
-    const uint32_t q = act ? eidx[s] : 0u;
-    float3 ra = make_float3(0.f, 0.f, 0.f), rb = make_float3(0.f, 0.f, 0.f);
-    if (act) {
-        ra = rel_pos(eval_a[q], P);
-        if (SEG) rb = rel_pos(eval_b[q], P);
-    }
     const double invh = P->invh;
-    const double qx = (double)ra.x * invh, qy = (double)ra.y * invh, qz = (double)ra.z * invh;
-    const int i = (int)floor(qx), j = (int)floor(qy), k = (int)floor(qz);
     const uint32_t C = (uint32_t)n * n * n;
-    float ux = 0.f, uy = 0.f, uz = 0.f;
-    if (act && i >= 0 && i < n && j >= 0 && j < n && k >= 0 && k < n) {
-        const double tx = qx - 0.5, ty = qy - 0.5, tz = qz - 0.5;
-        const double fx0 = floor(tx), fy0 = floor(ty), fz0 = floor(tz);
-        const int i0 = (int)fx0, j0 = (int)fy0, k0 = (int)fz0;
-        const float fx = (float)(tx - fx0), fy = (float)(ty - fy0), fz = (float)(tz - fz0);
-#pragma unroll
-        for (int c = 0; c < 8; c++) {
-            const int ii = i0 + (c & 1), jj = j0 + ((c >> 1) & 1), kk = k0 + (c >> 2);
-            const float wgt = ((c & 1) ? fx : 1.f - fx) * ((c & 2) ? fy : 1.f - fy) * ((c & 4) ? fz : 1.f - fz);
-            if (ii >= 0 && ii < n && jj >= 0 && jj < n && kk >= 0 && kk < n) {
-                const size_t g = ((size_t)kk * n + jj) * n + ii;
-                ux = fmaf(far[g], wgt, ux);
-                uy = fmaf(far[C + g], wgt, uy);
-                uz = fmaf(far[2 * (size_t)C + g], wgt, uz);
-            }
-        }
-    }
     PairAcc acc;
-    PairAcc2 acc2;
-    float3 o_w = make_float3(0.f, 0.f, 0.f);
+    PairSums sums;
     // some pair can reach t = 2: the exp-form walk (its sums carry 4 pi)
     const bool tier0 = P->need_exp2 != 0;
     if (K >= 0) {
+        float3 ra = make_float3(0.f, 0.f, 0.f), rb = make_float3(0.f, 0.f, 0.f);
+        if (act) {
+            const uint32_t q = eidx[s];
+            ra = rel_pos(eval_a[q], P);
+            if (SEG) rb = rel_pos(eval_b[q], P);
+        }
+        const double qx = (double)ra.x * invh, qy = (double)ra.y * invh, qz = (double)ra.z * invh;
+        const int i = (int)floor(qx), j = (int)floor(qy), k = (int)floor(qz);
         // FOLD: coefficients carry 1/(4 pi a^3); otherwise they have unit
         // scale and the sums are scaled once per point below
         const float cr = P->cr_f, inv_a3 = P->inv_a3_f, inv4pia3 = FOLD ? P->inv4pia3_f : 1.0f;
@@ -532,13 +472,9 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
         xf.nl2a3 = make_float2(-1.4426950408889634f * inv_a3, -1.4426950408889634f * inv_a3);
         xf.tsmall = kExpSmallT;
         xf.r3small = 1.001f * kExpSmallT / inv_a3;
-        // warp origin of the packed accumulation: lane 0's position
-        const float3 o = make_float3(__shfl_sync(0xffffffffu, ra.x, 0), __shfl_sync(0xffffffffu, ra.y, 0),
-                                     __shfl_sync(0xffffffffu, ra.z, 0));
-        o_w = o;
-        // the warp's box: every active lane's box, widened by far more than
+        // the warp's box: every active target's box, widened by far more than
         // the rounding of these float bounds (2^-18 of the coordinates' size)
-        float3 blo, bhi;
+        float spread;  // largest extent of the targets
         {
             float lx = act ? ra.x : INFINITY, ly = act ? ra.y : INFINITY, lz = act ? ra.z : INFINITY;
             float hx = act ? ra.x : -INFINITY, hy = act ? ra.y : -INFINITY, hz = act ? ra.z : -INFINITY;
@@ -551,10 +487,19 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
                 hy = fmaxf(hy, __shfl_xor_sync(0xffffffffu, hy, s2));
                 hz = fmaxf(hz, __shfl_xor_sync(0xffffffffu, hz, s2));
             }
+            float3 o = make_float3(0.f, 0.f, 0.f);
+            if (lx <= hx) o = make_float3(0.5f * (lx + hx), 0.5f * (ly + hy), 0.5f * (lz + hz));
+            spread = fmaxf(hx - lx, fmaxf(hy - ly, hz - lz));
             const float mx = ldexpf(fabsf(lx) + fabsf(hx) + cr, -18), my = ldexpf(fabsf(ly) + fabsf(hy) + cr, -18),
                         mz = ldexpf(fabsf(lz) + fabsf(hz) + cr, -18);
-            blo = make_float3(lx - cr - mx, ly - cr - my, lz - cr - mz);
-            bhi = make_float3(hx + cr + mx, hy + cr + my, hz + cr + mz);
+            // exp form: records inside [lo + near, hi - near] may lie within
+            // a / 4 of a target (1 % margin on a / 4, far above the trigger's)
+            const float near = cr - (float)(0.2525 * P->a);
+            if (lane == 0) {
+                W.box.lo = make_float4(lx - cr - mx, ly - cr - my, lz - cr - mz, near);
+                W.box.hi = make_float4(hx + cr + mx, hy + cr + my, hz + cr + mz, 0.f);
+                W.box.mid = make_float4(o.x, o.y, o.z, 0.f);
+            }
         }
         const float2 inv_a3_2 = make_float2(inv_a3, inv_a3);
         // The reference walks hash cells [i-K-1, i+K+1]^3.  Only the half-cells
@@ -592,10 +537,6 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
         // than half a cell, which the rounding bound prune_cells < 1/4 (far
         // beyond float rounding of the relative coordinates) guarantees;
         // otherwise every lane takes its own walk below.
-        const float cr_lane = act ? cr : -1.0f;
-        // exp form: records inside [blo + dnear, bhi - dnear] may lie within
-        // a / 4 of a lane (1 % margin on a / 4, far above the trigger's)
-        const float dnear = cr - (float)(0.2525 * P->a);
         // Segments: the pair test on the other end only ever drops a vortex
         // that sits at this lane's other end (|rb - r_p|^2 < 1e-24).  Each lane
         // looks for them among the records of the hash cells its other end can
@@ -644,31 +585,119 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
             }
             seg_mode = __any_sync(0xffffffffu, found >= 2) ? 1 : (__any_sync(0xffffffffu, found == 1) ? 2 : 0);
         }
+        if (lane == 0) {
+            const int cx0 = ulo[0] >> 1;
+            W.box.cells = make_int4(cx0, ulo[1], ulo[2], ulo[0]);
+            W.box.size = make_int4((uhi[0] >> 1) - cx0 + 1, uhi[1] - ulo[1] + 1, uhi[2] - ulo[2] + 1, uhi[0]);
+        }
+        __syncwarp();
         auto uniform_walk = [&](auto deg, auto segc) {
             constexpr int D = decltype(deg)::value;
             constexpr int S = decltype(segc)::value;
             const float2 *cfd = D == 0 ? sc.p5 : (D == 7 ? sc.p7 : sc.p4);
             Ring ring;
-            for (int k2 = ulo[2]; k2 <= uhi[2]; k2++)
-                for (int j2 = ulo[1]; j2 <= uhi[1]; j2++)
-                    for (int i2 = ulo[0]; i2 <= uhi[0];) {
-                        // the two x-halves of a cell are adjacent runs: walk them as one
-                        const bool both = ((i2 & 1) == 0) && (i2 + 1 <= uhi[0]);
-                        const int ci = i2 >> 1, cj = j2 >> 1, ck = k2 >> 1;
-                        const uint32_t cell = ((uint32_t)ck * n + (uint32_t)cj) * n + (uint32_t)ci;
-                        const uint32_t k0 = (cell << 3) | ((uint32_t)(j2 & 1) << 1) | ((uint32_t)(k2 & 1) << 2) |
-                                            (uint32_t)(i2 & 1);
-                        const uint32_t cs = start[cell];
-                        const uint32_t ps = sub_start[k0], next = k0 + (both ? 2u : 1u);
-                        const uint32_t pe = (next & 7u) ? sub_start[next] : end[cell];
-                        i2 += both ? 2 : 1;
-                        if (cs == kEmpty || ps == pe) continue;
-                        stage_run<S, COUNT, FOLD, D>(vrec, valf, ps, pe, cr_lane, ra, rb, pstar, o, blo, bhi,
-                                                     dnear, inv_a3_2, cfd, sc.t7, inv4pia3, D == 7 && need_exp2, pk,
-                                                     lane, ring, acc2, xf);
+            // the targets against `recs` records of the ring from slot s0
+            auto block = [&](auto full, auto check, uint32_t s0, uint32_t recs) {
+                constexpr bool FULL = decltype(full)::value, CHECK = decltype(check)::value;
+                pair_block<S, COUNT, FOLD, D, FULL, CHECK>(W, s0, recs >> 1, act ? cr : -1.0f, ra, rb, pstar, inv_a3_2,
+                                                           cfd, sc.t7, inv4pia3, D == 7 && need_exp2, xf, sums);
+            };
+            // The runs of records, one per (cell, y and z halves): the two x
+            // halves of a cell are adjacent.  The lanes look up 32 runs at
+            // once, and the records of those runs, laid end to end, are taken
+            // 32 at a time, each lane finding its record's run by bisection
+            // of the running sum of lengths: short runs (a sparse scene has a
+            // record or none in most) fill the lanes as long ones do.
+            const int runs = W.box.size.x * W.box.size.y * W.box.size.z;
+            constexpr int kStep = SPLIT ? kEvalThreads : 32;  // SPLIT: the warps take turns
+            for (int base = SPLIT ? 32 * warp : 0; base < runs; base += kStep) {
+                const int id = base + lane;
+                uint32_t ps = 0, len = 0;
+                if (id < runs) {
+                    const int4 c0 = W.box.cells, sz = W.box.size;
+                    const int row = id / sz.x, ci = c0.x + (id - row * sz.x), k = row / sz.y;
+                    const int j2 = c0.y + (row - k * sz.y), k2 = c0.z + k;
+                    const uint32_t cell = ((uint32_t)(k2 >> 1) * n + (uint32_t)(j2 >> 1)) * n + (uint32_t)ci;
+                    const uint32_t k0 = (cell << 3) | ((uint32_t)(j2 & 1) << 1) | ((uint32_t)(k2 & 1) << 2);
+                    const uint32_t cs = start[cell];
+                    const uint2 st = *reinterpret_cast<const uint2 *>(sub_start + k0);
+                    const uint32_t after = (k0 & 7u) == 6u ? end[cell] : sub_start[k0 + 2];
+                    if (cs != kEmpty) {
+                        ps = 2 * ci >= c0.w ? st.x : st.y;
+                        len = (2 * ci + 1 <= sz.w ? after : st.y) - ps;
                     }
-            finish_ring<S, COUNT, FOLD, D>(cr_lane, ra, rb, pstar, inv_a3_2, cfd, sc.t7, inv4pia3,
-                                           D == 7 && need_exp2, pk, lane, ring, acc2, xf);
+                }
+                uint32_t incl = len;
+#pragma unroll
+                for (int w = 1; w < 32; w <<= 1) {
+                    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, w);
+                    if (lane >= w) incl += v;
+                }
+                const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+                const uint32_t shift = ps - (incl - len);  // record = shift of its run + its place
+                for (uint32_t at = 0; at < total; at += 32) {
+                    const uint32_t place = at + (uint32_t)lane;
+                    int run = 0;
+#pragma unroll
+                    for (int w = 16; w > 0; w >>= 1)
+                        if (__shfl_sync(0xffffffffu, incl, run + w - 1) <= place) run += w;
+                    const uint32_t rec = __shfl_sync(0xffffffffu, shift, run & 31) + place;
+                    // the strength is loaded with the position (one latency
+                    // per chunk, not two), also for records the box tests drop
+                    float4 r = make_float4(INFINITY, 0.f, 0.f, 0.f), al = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (place < total) {
+                        r = vrec[rec];
+                        al = valf[rec];
+                    }
+                    // records outside the warp's box cannot pass any target's
+                    // test
+                    const float4 blo = W.box.lo, bhi = W.box.hi;
+                    const bool keep = r.x >= blo.x && r.x <= bhi.x && r.y >= blo.y && r.y <= bhi.y && r.z >= blo.z &&
+                                      r.z <= bhi.z;
+                    const unsigned kept = __ballot_sync(0xffffffffu, keep);
+                    if (kept == 0u) continue;
+                    // exp form: a record farther than that inside the box on
+                    // some axis is more than a / 4 (with a margin) from every
+                    // target, so no pair with it needs the small-t polynomial;
+                    // a block without another record skips the warp's test
+                    bool near_chunk = D != 0;
+                    if (D == 0) {
+                        const bool nr = keep && r.x >= blo.x + blo.w && r.x <= bhi.x - blo.w && r.y >= blo.y + blo.w &&
+                                        r.y <= bhi.y - blo.w && r.z >= blo.z + blo.w && r.z <= bhi.z - blo.w;
+                        near_chunk = __any_sync(0xffffffffu, nr);
+                    }
+                    if (keep) {
+                        const float4 o = W.box.mid;
+                        const uint32_t e = ring.fill + (uint32_t)__popc(kept & ((1u << lane) - 1u));
+                        stage_record(W, e, r, al, make_float3(o.x, o.y, o.z), rec);
+                    }
+                    ring.fill += (uint32_t)__popc(kept);
+                    ring.near = ring.near || near_chunk;
+                    // The ring never overwrites a record still waiting: before
+                    // a chunk fewer than 32 wait, a chunk adds at most 32, and
+                    // it holds 64.  The records still waiting after a block all
+                    // come from the chunk just staged, so its flag carries over.
+                    if (ring.fill - ring.head >= kBlockRecs) {
+                        __syncwarp();
+                        const uint32_t s0 = (ring.head >> 1) & (kRingSlots - 1);
+                        if (D != 0 || ring.near) block(std::true_type{}, std::true_type{}, s0, kBlockRecs);
+                        else block(std::true_type{}, std::false_type{}, s0, kBlockRecs);
+                        ring.head += kBlockRecs;
+                        ring.near = near_chunk && ring.fill != ring.head;
+                        __syncwarp();  // the next records may take the slots just read
+                    }
+                }
+            }
+            // what is left (fewer than 32), an odd record paired with one outside
+            // every box and without strength
+            const uint32_t rem = ring.fill - ring.head;
+            if (rem != 0) {
+                if (lane == 0 && (rem & 1u))
+                    stage_record(W, ring.fill, make_float4(-1e18f, -1e18f, -1e18f, 0.f),
+                                 make_float4(0.f, 0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f), 0xFFFFFFFEu);
+                __syncwarp();
+                block(std::false_type{}, std::true_type{}, (ring.head >> 1) & (kRingSlots - 1), rem + (rem & 1u));
+            }
         };
         auto walk = [&](auto deg) {
             if constexpr (SEG) {
@@ -679,27 +708,89 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
                 uniform_walk(deg, std::integral_constant<int, 0>{});
             }
         };
-        if (vol > 0 && vol <= kUniformMaxSub && P->prune_cells < 0.25) {
+        const bool close = !(spread > (float)(kMaxSpread / invh));
+        if (vol > 0 && vol <= kUniformMaxSub && close && P->prune_cells < 0.25) {
             if (tier0) walk(std::integral_constant<int, 0>{});
             else if (tier7) walk(std::integral_constant<int, 7>{});
             else walk(std::integral_constant<int, 4>{});
-        } else if (act && lo[0] <= hi[0]) {
-            // scattered warp (points outside the grid, sparse regions): own walk
-            for (int kk = lo[2] >> 1; kk <= (hi[2] >> 1); kk++)
-                for (int jj = lo[1] >> 1; jj <= (hi[1] >> 1); jj++)
-                    for (int ii = lo[0] >> 1; ii <= (hi[0] >> 1); ii++) {
-                        const uint32_t cell = ((uint32_t)kk * n + (uint32_t)jj) * n + (uint32_t)ii;
-                        const uint32_t ps = start[cell];
-                        if (ps == kEmpty) continue;
-                        cell_pairs<SEG, COUNT>(vrec, valf, ps, end[cell], true, ra, rb, cr, inv_a3, cf, inv4pia3, need_exp, acc);
-                    }
+        } else if (act && lo[0] <= hi[0] && lo[1] <= hi[1] && lo[2] <= hi[2]) {
+            // scattered warp (points outside the grid, sparse regions): own
+            // walk, by rows of cells, whose records are consecutive (SPLIT:
+            // the warps take the rows in turn)
+            const int x0 = lo[0] >> 1, x1 = hi[0] >> 1, y0 = lo[1] >> 1, z0 = lo[2] >> 1;
+            const int ny = (hi[1] >> 1) - y0 + 1, rows = ny * ((hi[2] >> 1) - z0 + 1);
+            for (int row = SPLIT ? warp : 0; row < rows; row += SPLIT ? kEvalThreads / 32 : 1) {
+                const int jj = y0 + row % ny, kk = z0 + row / ny;
+                const uint32_t cell = ((uint32_t)kk * n + (uint32_t)jj) * n;
+                uint32_t ps = kEmpty, pe = 0;
+                for (int ii = x0; ii <= x1; ii++) {
+                    const uint32_t cs = start[cell + ii];
+                    if (cs == kEmpty) continue;
+                    ps = min(ps, cs);
+                    pe = end[cell + ii];
+                }
+                if (ps == kEmpty) continue;
+                cell_pairs<SEG, COUNT>(vrec, valf, ps, pe, true, ra, rb, cr, inv_a3, cf, inv4pia3, need_exp, acc);
+            }
         }
     }
-    if (act) {
-        // packed walk: A x (ra - o) - B
-        const float Ax = acc2.ax.x + acc2.ax.y, Ay = acc2.ay.x + acc2.ay.y, Az = acc2.az.x + acc2.az.y;
-        const float Bx = acc2.bx.x + acc2.bx.y, By = acc2.by.x + acc2.by.y, Bz = acc2.bz.x + acc2.bz.y;
-        const float sx = ra.x - o_w.x, sy = ra.y - o_w.y, sz = ra.z - o_w.z;
+    float ab[6] = {sums.ax.x + sums.ax.y, sums.ay.x + sums.ay.y, sums.az.x + sums.az.y,
+                   sums.bx.x + sums.bx.y, sums.by.x + sums.by.y, sums.bz.x + sums.bz.y};
+    float ox = 0.f, oy = 0.f, oz = 0.f;
+    if (K >= 0) {
+        __syncwarp();
+        ox = W.box.mid.x;
+        oy = W.box.mid.y;
+        oz = W.box.mid.z;
+    }
+    if constexpr (SPLIT) {
+        // the four warps' sums, added in order
+        __syncthreads();  // the rings are done with
+        float *part = reinterpret_cast<float *>(stage) + lane;
+#pragma unroll
+        for (int q = 0; q < 9; q++)
+            part[(9 * warp + q) * 32] = q < 6 ? ab[q] : (q == 6 ? acc.x : (q == 7 ? acc.y : acc.z));
+        __syncthreads();
+        if (warp == 0) {
+            for (int w = 1; w < kEvalThreads / 32; w++) {
+                const float *from = part + 9 * w * 32;
+#pragma unroll
+                for (int q = 0; q < 6; q++) ab[q] += from[q * 32];
+                acc.x += from[6 * 32];
+                acc.y += from[7 * 32];
+                acc.z += from[8 * 32];
+            }
+        }
+    }
+    if (!COUNT && (!act || (SPLIT && warp != 0))) return;
+    // the far field, after the walk: its registers are the pair block's then
+    // (the point is read again)
+    const uint32_t q = act ? __ldcg(eidx + s) : 0u;
+    float3 ra = make_float3(0.f, 0.f, 0.f);
+    if (act) ra = rel_pos(eval_a[q], P);
+    float ux = 0.f, uy = 0.f, uz = 0.f;
+    const double qx = (double)ra.x * invh, qy = (double)ra.y * invh, qz = (double)ra.z * invh;
+    const int i = (int)floor(qx), j = (int)floor(qy), k = (int)floor(qz);
+    if (i >= 0 && i < n && j >= 0 && j < n && k >= 0 && k < n) {
+        const double tx = qx - 0.5, ty = qy - 0.5, tz = qz - 0.5;
+        const double fx0 = floor(tx), fy0 = floor(ty), fz0 = floor(tz);
+        const int i0 = (int)fx0, j0 = (int)fy0, k0 = (int)fz0;
+        const float fx = (float)(tx - fx0), fy = (float)(ty - fy0), fz = (float)(tz - fz0);
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            const int ii = i0 + (c & 1), jj = j0 + ((c >> 1) & 1), kk = k0 + (c >> 2);
+            const float wgt = ((c & 1) ? fx : 1.f - fx) * ((c & 2) ? fy : 1.f - fy) * ((c & 4) ? fz : 1.f - fz);
+            if (ii >= 0 && ii < n && jj >= 0 && jj < n && kk >= 0 && kk < n) {
+                const size_t g = ((size_t)kk * n + jj) * n + ii;
+                ux = fmaf(far[g], wgt, ux);
+                uy = fmaf(far[C + g], wgt, uy);
+                uz = fmaf(far[2 * (size_t)C + g], wgt, uz);
+            }
+        }
+    }
+    if (act && (!SPLIT || warp == 0)) {
+        const float Ax = ab[0], Ay = ab[1], Az = ab[2], Bx = ab[3], By = ab[4], Bz = ab[5];
+        const float sx = ra.x - ox, sy = ra.y - oy, sz = ra.z - oz;
         if (tier0) {
             // exp-form sums carry 4 pi (the reference's literal); the lane's
             // own walk carries the scale of its coefficients
@@ -738,18 +829,20 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
         }
     }
     if (COUNT) {
-        unsigned long long pairs = acc.n + acc2.n;
+        unsigned long long pairs = acc.n + sums.n;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
         if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(pair_count, pairs);
     }
 }
 
-// One scene: block b evaluates points [128 b, 128 b + 128) of the order.
-template <bool SEG, bool COUNT, bool FOLD>
-__global__ void __launch_bounds__(kEvalThreads, kEvalBlocksPerSM) eval_kernel(const SmoothSeries sc, const EvalArgs ea) {
-    __shared__ float4 stage[(kEvalThreads / 32) * kPackPlanes * kPackSlots];
-    eval_points<SEG, COUNT, FOLD>(sc, ea, blockIdx.x, stage);
+// One scene: block b evaluates points [128 b, 128 b + 128) of the order, or
+// (SPLIT) [32 b, 32 b + 32).
+template <bool SEG, bool COUNT, bool FOLD, bool SPLIT>
+__global__ void __launch_bounds__(kEvalThreads, kEvalBlocksPerSM)
+eval_kernel(const SmoothSeries sc, const EvalArgs ea) {
+    __shared__ WarpMem stage[kEvalThreads / 32];
+    eval_points<SEG, COUNT, FOLD, SPLIT>(sc, ea, blockIdx.x, stage);
 }
 
 // Several scenes in one launch: block b takes work item work[b] = (scene,
@@ -757,15 +850,15 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalBlocksPerSM) eval_kernel(co
 // scenes with the most pairs per point come first, which the block scheduler
 // then hands out first (longest work first); each point's arithmetic is the
 // one-scene kernel's, so results do not depend on the batch.
-template <bool SEG, bool COUNT, bool FOLD>
+template <bool SEG, bool COUNT, bool FOLD, bool SPLIT>
 __global__ void __launch_bounds__(kEvalThreads, kEvalBlocksPerSM)
 eval_batch_kernel(const SmoothSeries sc, const EvalArgs *__restrict__ scenes, const uint2 *__restrict__ work) {
-    __shared__ float4 stage[(kEvalThreads / 32) * kPackPlanes * kPackSlots];
+    __shared__ WarpMem stage[kEvalThreads / 32];
     __shared__ EvalArgs sa;  // the block's scene, read from shared memory where used
     const uint2 it = work[blockIdx.x];
     if (threadIdx.x == 0) sa = scenes[it.x];
     __syncthreads();
-    eval_points<SEG, COUNT, FOLD>(sc, sa, it.y, stage);
+    eval_points<SEG, COUNT, FOLD, SPLIT>(sc, sa, it.y, stage);
 }
 
 // Monomial coefficients of the degree-deg polynomial that interpolates
@@ -804,12 +897,13 @@ cudaError_t launch_eval_sort(pppm_scene *s, const float4 *eval_a, uint32_t M) {
     uint32_t *skey = nullptr, *sidx = nullptr;
     prof_begin(s, kStageEvalSort);
     ::pppm::note_launch();
-    // quarter-cell order while the key fits 32 bits (n <= 256), else octants
-    const int fine = (64ull * s->C < (1ull << 32)) ? 1 : 0;
-    eval_keys_kernel<<<(M + 255) / 256, 256, 0, s->stream>>>(eval_a, M, s->dparams, fine, s->ekey[0], s->eidx[0]);
+    const int per_cell = s->n <= 256 ? 4 : 2;
+    int side = 1;
+    while ((1u << side) < s->n * (uint32_t)per_cell) side++;
+    eval_keys_kernel<<<(M + 255) / 256, 256, 0, s->stream>>>(eval_a, M, s->dparams, per_cell, side, s->ekey[0],
+                                                             s->eidx[0]);
     PPPM_CUDA_TRY(cudaGetLastError());
-    uint32_t bits = 1;
-    while (bits < 32 && (1ull << bits) <= (fine ? 64ull : 8ull) * s->C) bits++;
+    const uint32_t bits = 3u * (uint32_t)side;
     PPPM_CUDA_TRY(radix_sort_pairs(s->stream, M, bits, s->ekey, s->eidx, s->hist, &skey, &sidx));
     prof_end(s, kStageEvalSort);
     s->esorted_idx = sidx;
@@ -882,6 +976,24 @@ static EvalArgs make_args(pppm_scene *s, const float4 *eval_a, const float4 *eva
     return a;
 }
 
+// Whether a scene's points are evaluated 32 to a block, its four warps sharing
+// their walk: with fewer than about two warps of points for each that the GPU
+// holds, the longest walks (the densest part of a scene) set the time, and a
+// quarter of a walk is what each warp then does (65,537 points, K = 3: 5.6 ms
+// without, 2.6 ms with it).
+constexpr uint32_t kSplitMaxPoints = 2 * 148 * kEvalBlocksPerSM * kEvalThreads;
+static bool eval_split(uint32_t M) { return M <= kSplitMaxPoints; }
+uint32_t eval_blocks(uint32_t M) {
+    const uint32_t per = eval_split(M) ? 32 : kEvalThreads;
+    return (M + per - 1) / per;
+}
+
+template <class F>
+static void pick(bool v, F f) {
+    if (v) f(std::true_type{});
+    else f(std::false_type{});
+}
+
 cudaError_t launch_eval(pppm_scene *s, const float4 *eval_a, const float4 *eval_b, int is_segment, uint32_t M,
                         double *u, double *v, double *w, float *uf, int count_pairs) {
     PPPM_CUDA_TRY(launch_eval_sort(s, eval_a, M));
@@ -889,23 +1001,21 @@ cudaError_t launch_eval(pppm_scene *s, const float4 *eval_a, const float4 *eval_
     prof_begin(s, kStageEval);
     ::pppm::note_launch();
     const bool seg = (is_segment == 1) && (eval_b != eval_a);
-    const unsigned grid = (M + kEvalThreads - 1) / kEvalThreads;
+    const bool split = eval_split(M);
+    const unsigned grid = eval_blocks(M);
     SmoothSeries sc;
     const bool fold = make_series(s, sc);
     const EvalArgs ea = make_args(s, eval_a, eval_b, M, u, v, w, uf, count_pairs ? s->pair_count : nullptr);
-#define PPPM_EVAL_LAUNCH(SEG_, COUNT_)                                                              \
-    do {                                                                                              \
-        if (fold) eval_kernel<SEG_, COUNT_, true><<<grid, kEvalThreads, 0, s->stream>>>(sc, ea);      \
-        else eval_kernel<SEG_, COUNT_, false><<<grid, kEvalThreads, 0, s->stream>>>(sc, ea);         \
-    } while (0)
-    if (seg) {
-        if (count_pairs) PPPM_EVAL_LAUNCH(true, true);
-        else PPPM_EVAL_LAUNCH(true, false);
-    } else {
-        if (count_pairs) PPPM_EVAL_LAUNCH(false, true);
-        else PPPM_EVAL_LAUNCH(false, false);
-    }
-#undef PPPM_EVAL_LAUNCH
+    pick(seg, [&](auto a) {
+        pick(count_pairs != 0, [&](auto b) {
+            pick(fold, [&](auto c) {
+                pick(split, [&](auto d) {
+                    eval_kernel<decltype(a)::value, decltype(b)::value, decltype(c)::value, decltype(d)::value>
+                        <<<grid, kEvalThreads, 0, s->stream>>>(sc, ea);
+                });
+            });
+        });
+    });
     prof_end(s, kStageEval);
     return cudaGetLastError();
 }
@@ -921,6 +1031,7 @@ cudaError_t eval_batch_prepare(pppm_scene *s, const float4 *eval_a, const float4
     static_assert(sizeof(SmoothSeries) <= sizeof(mode->series), "series bytes");
     memcpy(mode->series, &sc, sizeof(sc));
     mode->seg = (is_segment == 1) && (eval_b != eval_a);
+    mode->split = eval_split(M);
     *args = make_args(s, eval_a, eval_b, M, u, v, w, nullptr, nullptr);
     return cudaSuccess;
 }
@@ -933,13 +1044,14 @@ cudaError_t launch_eval_batch(const EvalMode &mode, const EvalArgs *args_dev, co
     SmoothSeries sc;
     memcpy(&sc, mode.series, sizeof(sc));
     ::pppm::note_launch();
-    if (mode.seg) {
-        if (mode.fold) eval_batch_kernel<true, false, true><<<blocks, kEvalThreads, 0, st>>>(sc, args_dev, work_dev);
-        else eval_batch_kernel<true, false, false><<<blocks, kEvalThreads, 0, st>>>(sc, args_dev, work_dev);
-    } else {
-        if (mode.fold) eval_batch_kernel<false, false, true><<<blocks, kEvalThreads, 0, st>>>(sc, args_dev, work_dev);
-        else eval_batch_kernel<false, false, false><<<blocks, kEvalThreads, 0, st>>>(sc, args_dev, work_dev);
-    }
+    pick(mode.seg, [&](auto a) {
+        pick(mode.fold, [&](auto c) {
+            pick(mode.split, [&](auto d) {
+                eval_batch_kernel<decltype(a)::value, false, decltype(c)::value, decltype(d)::value>
+                    <<<blocks, kEvalThreads, 0, st>>>(sc, args_dev, work_dev);
+            });
+        });
+    });
     return cudaGetLastError();
 }
 

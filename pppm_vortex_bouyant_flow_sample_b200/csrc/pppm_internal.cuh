@@ -300,10 +300,10 @@ struct EvalArgs {
 // What items of one batched evaluation launch must share: the smoothing
 // series (bytes), its folding and the segment mode.
 struct EvalMode {
-    bool fold = false, seg = false;
+    bool fold = false, seg = false, split = false;
     unsigned char series[192] = {};
     bool same(const EvalMode &o) const {
-        if (fold != o.fold || seg != o.seg) return false;
+        if (fold != o.fold || seg != o.seg || split != o.split) return false;
         for (int i = 0; i < 192; i++)
             if (series[i] != o.series[i]) return false;
         return true;
@@ -311,6 +311,7 @@ struct EvalMode {
 };
 cudaError_t eval_batch_prepare(pppm_scene *s, const float4 *eval_a, const float4 *eval_b, int is_segment, uint32_t M,
                                double *u, double *v, double *w, EvalArgs *args, EvalMode *mode);
+uint32_t eval_blocks(uint32_t M);  // blocks of the evaluation of M points
 cudaError_t launch_eval_batch(const EvalMode &mode, const EvalArgs *args_dev, const uint2 *work_dev, uint32_t blocks,
                               cudaStream_t st);
 cudaError_t launch_gather_sorted(pppm_scene *s, float4 *pos_out, double *alpha_out);

@@ -1,6 +1,7 @@
 """The particle kernels at the sizes where their paths change: the sort in one
-block and in tiles, and the deposit of cells with very different numbers of
-vortices."""
+block and in tiles, the evaluation's warps and blocks
+(one block's four warps share 32 points below a size), its dense and sparse
+walks, and the deposit's cells."""
 import numpy as np
 import pytest
 
@@ -51,6 +52,53 @@ def test_sort_is_stable_at_every_size(pb, n, N):
     order = np.argsort(want, kind="stable")
     assert np.array_equal(idx, order)
     assert np.array_equal(key, want[order])
+
+
+@pytest.mark.parametrize("K", [0, 1, 3])
+@pytest.mark.parametrize("a_cells", [0.0, 1.0])
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 32, 33, 129, 700])
+def test_evaluation_of_few_points(pb, oracle, M, a_cells, K):
+    """Ragged groups, warps and blocks of targets in a dense part of a scene (45
+    vortices a cell), with the smoothing polynomial (a = 0.3 is 5 cells) and
+    the exp form; the pair count leaves out lanes without a point."""
+    rng = np.random.default_rng(M)
+    N = 20000
+    pos, al = _points(rng, N, 0.3, 0.7), rng.normal(size=(N, 3))
+    ev = _points(rng, M, 0.25, 0.75)
+    scene = pb.Scene(16, K=K, a=0.3, a_cells=a_cells, cap_vort=N, cap_eval=M, domain="fixed", **BOX)
+    scene.set_vortices(_dev(pos), _dev(al.T))
+    scene.build_far_field()
+    u = scene.eval(_dev(ev)).cpu().numpy()
+    pairs = scene.count_pairs(_dev(ev))
+    a = scene.smoothing()
+    scene.close()
+    ref, d = oracle.pppm(oracle.params(16, K=K, a=a, domain_mode=1, **BOX), pos, al, ev, None, 0, dump=True)
+    assert pairs == int(d["pairs"][0])
+    assert rel_l2(u, ref) <= 1e-5
+
+
+@pytest.mark.parametrize("per_cell", [0.3, 2.0, 6.0, 20.0])
+@pytest.mark.parametrize("seg", [0, 1])
+def test_evaluation_from_sparse_to_dense(pb, oracle, per_cell, seg):
+    """Groups of targets that span several cells walk their own boxes, dense
+    ones the shared walk, with and without a segment's other end."""
+    rng = np.random.default_rng(7)
+    n = 24
+    N = int(per_cell * (n - 4) ** 3)
+    pos, al = _points(rng, N, 2.0 / n, 1.0 - 2.0 / n), rng.normal(size=(N, 3))
+    other = pos.copy()
+    ev = pos.copy()
+    if seg:
+        ev[:, :3] += rng.normal(0.0, 0.1 / n, (N, 3)).astype(np.float32)
+    sub = np.sort(rng.choice(N, min(N, 3000), replace=False))
+    scene = pb.Scene(n, a_cells=1.0, cap_vort=N, cap_eval=N, domain="fixed", **BOX)
+    scene.set_vortices(_dev(pos), _dev(al.T))
+    scene.build_far_field()
+    u = scene.eval(_dev(ev), _dev(other), 1).cpu().numpy()
+    scene.close()
+    ref = oracle.pppm(oracle.params(n, a=float(np.float32(1.0 / n)), domain_mode=1, **BOX), pos, al, ev[sub],
+                      other[sub], 1)[0]
+    assert rel_l2(u[sub], ref) <= 1e-5
 
 
 def test_deposit_of_uneven_cells(pb, oracle):
