@@ -241,9 +241,9 @@ pppm_status pppm_get_stage_times(pppm_scene *s, double *ms, int cap, int *count)
 /* Number of kernels this library has launched in the process so far. */
 uint64_t pppm_kernel_launches(void);
 /* The multigrid smoother's autotuner (no reference counterpart).  By default
- * every level runs the plain red-black half sweeps.  With PPPM_MG_TB=auto in
- * the environment when a scene or multigrid object is created, each level of
- * edge >= 256 runs either the sweep kernel or one of the temporally
+ * every level of edge > 32 runs one launch per red-black sweep.  With
+ * PPPM_MG_TB=auto in the environment when a scene or multigrid object is
+ * created, each level of edge >= 256 runs either that or one of the temporally
  * blocked variants (T half sweeps per pass, TX x TY tiles, TMA plane
  * staging), whichever measured fastest for that edge and component count on
  * this device; PPPM_MG_TB=<index> forces one variant.  Every choice gives the
