@@ -12,7 +12,7 @@ from __future__ import annotations
 import json
 import os
 
-# directories of the sources that the checkers are compiled from
+# directories that have to be there
 _PARTS = ("hybridFastSummation", "particle_hash", "multigrid", "Particle_renderer")
 _REPO = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
