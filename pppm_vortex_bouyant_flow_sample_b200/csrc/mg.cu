@@ -405,7 +405,9 @@ static cudaError_t add_to_psi(const MGPlan &m, double *psi, bool set_psi) {
 // The cycle's x at `level` starts at zero plus, when xc is set, the injected
 // correction from level + 1 (the full multigrid's prolongation); the coarser
 // levels start at zero as the reference zeroes them.  The result is left in
-// lv[level].x, or with psi (level 0) added to it or stored in it instead.  The
+// lv[level].x, or with psi (level 0) added to it or stored in it instead: by
+// the last sweep, which takes psi 16 bytes at a time, or by a kernel of its own
+// where psi is the caller's array and need only be aligned as a double.  The
 // levels from mg_tail_level on run in one launch.
 static cudaError_t vcycle32(const MGPlan &m, int level, const float *xc = nullptr, double *psi = nullptr,
                             bool set_psi = false) {
@@ -419,6 +421,7 @@ static cudaError_t vcycle32(const MGPlan &m, int level, const float *xc = nullpt
         return psi ? add_to_psi(m, psi, set_psi) : cudaSuccess;
     }
     const int T = mg_tail_level(m);
+    const bool aligned = reinterpret_cast<uintptr_t>(psi) % 16 == 0;
     XAt at[kMaxLevels];
     for (int j = level; j < T; j++) {
         PPPM_CUDA_TRY(smooth(m, j, kXZero, j == level ? xc : nullptr, &at[j]));
@@ -427,7 +430,7 @@ static cudaError_t vcycle32(const MGPlan &m, int level, const float *xc = nullpt
     }
     PPPM_CUDA_TRY(mg_tail_launch(m, std::max(T, level), kTailCycle));
     for (int j = T - 1; j >= level; j--) {
-        const bool last = j == 0 && psi && !tb_level(m, j);
+        const bool last = j == 0 && psi && aligned && !tb_level(m, j);
         XAt res;
         PPPM_CUDA_TRY(smooth(m, j, at[j], m.lv[j + 1].x, &res, last ? psi : nullptr, set_psi));
         if (last) return cudaSuccess;

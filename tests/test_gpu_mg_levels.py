@@ -49,6 +49,28 @@ def test_full_multigrid_and_vcycle(pb, oracle, n):
     mg.m_FinalMemoryEachLevel()
 
 
+@pytest.mark.parametrize("n", [16, 32, 40, 64])
+def test_vcycle_of_a_slice_at_an_odd_offset(pb, oracle, n):
+    """x and b need only be aligned as doubles: edges whose last sweep adds to
+    x by pairs of doubles (above 32) and edges that end in the cluster launch."""
+    import torch
+    rng = np.random.default_rng(n)
+    x0, b = rng.standard_normal(n ** 3), rng.standard_normal(n ** 3)
+    buf = torch.full((n ** 3 + 2,), 7.0, dtype=torch.float64, device="cuda")
+    x = buf[1:-1]
+    x.copy_(torch.from_numpy(x0))
+    bb = torch.zeros(n ** 3 + 1, dtype=torch.float64, device="cuda")[1:]
+    bb.copy_(torch.from_numpy(b))
+    assert x.data_ptr() % 16 == 8 and bb.data_ptr() % 16 == 8
+    mg = pb.MultiGridSolver3DPeriod_double()
+    mg.m_InitialSystem(n, n, n)
+    mg.m_Vcycle(x, bb)
+    ref = oracle.mg_vcycle(x0, b, n)
+    assert np.linalg.norm(x.cpu().numpy() - ref) <= 6e-6 * np.linalg.norm(ref - x0)
+    assert buf[0].item() == 7.0 and buf[-1].item() == 7.0
+    mg.m_FinalMemoryEachLevel()
+
+
 @pytest.mark.parametrize("tol", [1e-6, 1e-10])
 @pytest.mark.parametrize("n", [12, 16, 20, 28, 32, 40, 64, 112])
 def test_corrected_cycles_reach_the_tolerance(pb, oracle, n, tol):
