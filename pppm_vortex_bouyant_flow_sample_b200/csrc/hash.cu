@@ -208,24 +208,28 @@ __global__ void keys_explicit_kernel(const float4 *__restrict__ pos, uint32_t N,
     idx[t] = t;
 }
 
-// Per-tile digit histogram, written digit-major: hist[d * nb + b].
+// Per-tile digit histogram, written digit-major: hist[d * nb + b], counted in
+// shared memory by the whole block.  Keys come four at a time where their
+// address allows it; pppm_spatial_hash_noalloc sorts in its caller's arrays,
+// which need only be aligned as words.
 __global__ void __launch_bounds__(kRsThreads)
 radix_upsweep_kernel(const uint32_t *__restrict__ keys, uint32_t N, int shift, uint32_t *__restrict__ hist) {
     __shared__ uint32_t cnt[256];
     cnt[threadIdx.x] = 0;
     __syncthreads();
     const uint32_t base = blockIdx.x * kRsTile;
+    const bool aligned = reinterpret_cast<uintptr_t>(keys) % sizeof(uint4) == 0;
     uint4 k[kRsItems / 4];
 #pragma unroll
     for (int j = 0; j < kRsItems / 4; j++) {
         const uint32_t i = base + 4 * (j * kRsThreads + threadIdx.x);
-        if (i + 3 < N) {
+        if (aligned && i + 3 < N) {
             k[j] = *reinterpret_cast<const uint4 *>(keys + i);
         } else {
             k[j].x = i < N ? keys[i] : 0u;
             k[j].y = i + 1 < N ? keys[i + 1] : 0u;
             k[j].z = i + 2 < N ? keys[i + 2] : 0u;
-            k[j].w = 0u;
+            k[j].w = i + 3 < N ? keys[i + 3] : 0u;
         }
     }
 #pragma unroll

@@ -64,9 +64,9 @@ def _copy_dev(torch, dst, src_ptr, count):
     dst.copy_(torch.as_tensor(View(), device="cuda"))
 
 
-def _noalloc(lib, torch, pos, n, h, origin):
+def _noalloc(lib, torch, pos, n, h, origin, offset=0):
     N = pos.shape[0]
-    outs = [torch.full((c,), -7, dtype=torch.int32, device="cuda") for c in (N, N, n ** 3, n ** 3)]
+    outs = [torch.full((c + offset,), -7, dtype=torch.int32, device="cuda")[offset:] for c in (N, N, n ** 3, n ** 3)]
     o = (C.c_float * 3)(*origin)
     rc = lib.pppm_spatial_hash_noalloc(N, C.c_void_p(pos.data_ptr()), n, C.c_float(h), o,
                                        *[C.c_void_p(t.data_ptr()) for t in outs], None)
@@ -90,6 +90,23 @@ def test_noalloc_matches_allocating_hash_twice(env, n):
         ref = _reference_tables(lib, torch, pos, n, h, origin)
         for g, r, name in zip(got, ref, ("sorted_key", "sorted_idx", "cell_start", "cell_end")):
             assert np.array_equal(g, r), name
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3])
+@pytest.mark.parametrize("n,N", [(16, 8193), (64, 20_001), (64, 65_536)])
+def test_noalloc_into_arrays_aligned_as_words(env, n, N, offset):
+    """The output arrays, in which the sort's passes also run, may start at any
+    word: two and three passes (the caller's keys are the first or the second
+    pass's input), a tile of one key and whole tiles."""
+    lib, torch = env
+    pos = torch.zeros((N, 4), dtype=torch.float32, device="cuda")
+    rng = np.random.default_rng(N)
+    pos[:, :3] = torch.from_numpy(rng.random((N, 3), dtype=np.float32)).cuda()
+    h, origin = 1.3 / n, (0.05, 0.02, 0.08)
+    got = _noalloc(lib, torch, pos, n, h, origin, offset)
+    ref = _reference_tables(lib, torch, pos, n, h, origin)
+    for g, r, name in zip(got, ref, ("sorted_key", "sorted_idx", "cell_start", "cell_end")):
+        assert np.array_equal(g, r), name
 
 
 def test_noalloc_rejects_oversize_without_touching_gpu(env):
