@@ -200,7 +200,7 @@ constexpr uint32_t kBlockRecs = 32;  // records per block of the pair loop
 // the registers of the pair block.
 struct WarpBox {
     float4 lo, hi;   // the targets' boxes' union; lo.w: margin of the near test
-    float4 mid;      // origin of the moments
+    float4 mid;      // origin of the moments; w: the lanes with a near field, as bits
     int4 cells, size;  // first cell x, half-cells y, z and x; cells x, half-cells y, z and last half-cell x
 };
 struct WarpMem {
@@ -472,12 +472,46 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
         xf.nl2a3 = make_float2(-1.4426950408889634f * inv_a3, -1.4426950408889634f * inv_a3);
         xf.tsmall = kExpSmallT;
         xf.r3small = 1.001f * kExpSmallT / inv_a3;
-        // the warp's box: every active target's box, widened by far more than
-        // the rounding of these float bounds (2^-18 of the coordinates' size)
-        float spread;  // largest extent of the targets
+        const float2 inv_a3_2 = make_float2(inv_a3, inv_a3);
+        // The reference walks hash cells [i-K-1, i+K+1]^3.  Only the half-cells
+        // (cell, octant runs of the vortex order) that can hold a vortex inside
+        // the point's box are visited: the box spans K+0.5 cells either side,
+        // widened by the hash/NGP rounding bound.  Coordinates below are in
+        // half cells.
+        const double R = (double)K + 0.5 + P->prune_cells;
+        int lo[3], hi[3], rlo[3], rhi[3];
+        const double qq[3] = {qx, qy, qz};
+        const int cc[3] = {i, j, k};
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            rlo[a] = cc[a] - K - 1;
+            rhi[a] = cc[a] + K + 1;
+            lo[a] = max(max(2 * rlo[a], 0), (int)floor(2.0 * (qq[a] - R)));
+            hi[a] = min(min(2 * rhi[a] + 1, 2 * n - 1), (int)floor(2.0 * (qq[a] + R)));
+        }
+        // A target without a near field (outside the grid and its margin, at
+        // infinity, not a number) has no say in the warp's walk: it would
+        // stretch the others' box, and an infinite one would put their moments'
+        // origin at infinity.  It follows one of them through the walk, and its
+        // sums are dropped at the end (a mask of its own in the pair loop made
+        // the 1M ring's evaluation 1.5 % longer).
+        const bool box = act && lo[0] <= hi[0] && lo[1] <= hi[1] && lo[2] <= hi[2] && !isnan(ra.x + ra.y + ra.z);
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+            if (!box) { lo[a] = INT_MAX; hi[a] = INT_MIN; }
+        const unsigned near_lanes = __ballot_sync(0xffffffffu, box);
         {
-            float lx = act ? ra.x : INFINITY, ly = act ? ra.y : INFINITY, lz = act ? ra.z : INFINITY;
-            float hx = act ? ra.x : -INFINITY, hy = act ? ra.y : -INFINITY, hz = act ? ra.z : -INFINITY;
+            const int from = near_lanes ? __ffs(near_lanes) - 1 : 0;
+            const float3 other = make_float3(__shfl_sync(0xffffffffu, ra.x, from), __shfl_sync(0xffffffffu, ra.y, from),
+                                             __shfl_sync(0xffffffffu, ra.z, from));
+            if (!box) ra = other;
+        }
+        // the warp's box: every such target's box, widened by far more than
+        // the rounding of these float bounds (2^-18 of the coordinates' size)
+        float spread;  // largest extent of the targets (none: negative)
+        {
+            float lx = box ? ra.x : INFINITY, ly = box ? ra.y : INFINITY, lz = box ? ra.z : INFINITY;
+            float hx = box ? ra.x : -INFINITY, hy = box ? ra.y : -INFINITY, hz = box ? ra.z : -INFINITY;
 #pragma unroll
             for (int s2 = 16; s2 > 0; s2 >>= 1) {
                 lx = fminf(lx, __shfl_xor_sync(0xffffffffu, lx, s2));
@@ -498,26 +532,8 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
             if (lane == 0) {
                 W.box.lo = make_float4(lx - cr - mx, ly - cr - my, lz - cr - mz, near);
                 W.box.hi = make_float4(hx + cr + mx, hy + cr + my, hz + cr + mz, 0.f);
-                W.box.mid = make_float4(o.x, o.y, o.z, 0.f);
+                W.box.mid = make_float4(o.x, o.y, o.z, __uint_as_float(near_lanes));
             }
-        }
-        const float2 inv_a3_2 = make_float2(inv_a3, inv_a3);
-        // The reference walks hash cells [i-K-1, i+K+1]^3.  Only the half-cells
-        // (cell, octant runs of the vortex order) that can hold a vortex inside
-        // the point's box are visited: the box spans K+0.5 cells either side,
-        // widened by the hash/NGP rounding bound.  Coordinates below are in
-        // half cells.
-        const double R = (double)K + 0.5 + P->prune_cells;
-        int lo[3], hi[3], rlo[3], rhi[3];
-        const double qq[3] = {qx, qy, qz};
-        const int cc[3] = {i, j, k};
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            rlo[a] = cc[a] - K - 1;
-            rhi[a] = cc[a] + K + 1;
-            lo[a] = max(max(2 * rlo[a], 0), (int)floor(2.0 * (qq[a] - R)));
-            hi[a] = min(min(2 * rhi[a] + 1, 2 * n - 1), (int)floor(2.0 * (qq[a] + R)));
-            if (!act || lo[a] > hi[a]) { lo[a] = INT_MAX; hi[a] = INT_MIN; }
         }
         int ulo[3], uhi[3];
 #pragma unroll
@@ -550,7 +566,7 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
         uint32_t pstar = 0xFFFFFFFFu;
         if (SEG) {
             int found = 0;
-            if (act) {
+            if (box) {
                 const double pr = P->prune_cells + 1e-6;
                 const double qb[3] = {(double)rb.x * invh, (double)rb.y * invh, (double)rb.z * invh};
                 int clo[3], chi[3];
@@ -599,7 +615,7 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
             // the targets against `recs` records of the ring from slot s0
             auto block = [&](auto full, auto check, uint32_t s0, uint32_t recs) {
                 constexpr bool FULL = decltype(full)::value, CHECK = decltype(check)::value;
-                pair_block<S, COUNT, FOLD, D, FULL, CHECK>(W, s0, recs >> 1, act ? cr : -1.0f, ra, rb, pstar, inv_a3_2,
+                pair_block<S, COUNT, FOLD, D, FULL, CHECK>(W, s0, recs >> 1, (COUNT ? box : act) ? cr : -1.0f, ra, rb, pstar, inv_a3_2,
                                                            cfd, sc.t7, inv4pia3, D == 7 && need_exp2, xf, sums);
             };
             // The runs of records, one per (cell, y and z halves): the two x
@@ -713,10 +729,10 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
             if (tier0) walk(std::integral_constant<int, 0>{});
             else if (tier7) walk(std::integral_constant<int, 7>{});
             else walk(std::integral_constant<int, 4>{});
-        } else if (act && lo[0] <= hi[0] && lo[1] <= hi[1] && lo[2] <= hi[2]) {
-            // scattered warp (points outside the grid, sparse regions): own
-            // walk, by rows of cells, whose records are consecutive (SPLIT:
-            // the warps take the rows in turn)
+        } else if (box) {
+            // scattered warp (sparse regions): own walk, by rows of cells,
+            // whose records are consecutive (SPLIT: the warps take the rows
+            // in turn)
             const int x0 = lo[0] >> 1, x1 = hi[0] >> 1, y0 = lo[1] >> 1, z0 = lo[2] >> 1;
             const int ny = (hi[1] >> 1) - y0 + 1, rows = ny * ((hi[2] >> 1) - z0 + 1);
             for (int row = SPLIT ? warp : 0; row < rows; row += SPLIT ? kEvalThreads / 32 : 1) {
@@ -737,11 +753,13 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
     float ab[6] = {sums.ax.x + sums.ax.y, sums.ay.x + sums.ay.y, sums.az.x + sums.az.y,
                    sums.bx.x + sums.bx.y, sums.by.x + sums.by.y, sums.bz.x + sums.bz.y};
     float ox = 0.f, oy = 0.f, oz = 0.f;
+    bool near = false;
     if (K >= 0) {
         __syncwarp();
         ox = W.box.mid.x;
         oy = W.box.mid.y;
         oz = W.box.mid.z;
+        near = ((__float_as_uint(W.box.mid.w) >> lane) & 1u) != 0u;
     }
     if constexpr (SPLIT) {
         // the four warps' sums, added in order
@@ -791,23 +809,25 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
     if (act && (!SPLIT || warp == 0)) {
         const float Ax = ab[0], Ay = ab[1], Az = ab[2], Bx = ab[3], By = ab[4], Bz = ab[5];
         const float sx = ra.x - ox, sy = ra.y - oy, sz = ra.z - oz;
+        const float nx = near ? fmaf(Ay, sz, -(Az * sy)) - Bx : 0.f, ny = near ? fmaf(Az, sx, -(Ax * sz)) - By : 0.f,
+                    nz = near ? fmaf(Ax, sy, -(Ay * sx)) - Bz : 0.f;
         if (tier0) {
             // exp-form sums carry 4 pi (the reference's literal); the lane's
             // own walk carries the scale of its coefficients
             const float kown = FOLD ? 1.0f : P->inv4pia3_f;
             const float k4 = (float)(1.0 / kFourPi);
-            ux = fmaf(fmaf(Ay, sz, -(Az * sy)) - Bx, k4, fmaf(acc.x, kown, ux));
-            uy = fmaf(fmaf(Az, sx, -(Ax * sz)) - By, k4, fmaf(acc.y, kown, uy));
-            uz = fmaf(fmaf(Ax, sy, -(Ay * sx)) - Bz, k4, fmaf(acc.z, kown, uz));
+            ux = fmaf(nx, k4, fmaf(acc.x, kown, ux));
+            uy = fmaf(ny, k4, fmaf(acc.y, kown, uy));
+            uz = fmaf(nz, k4, fmaf(acc.z, kown, uz));
         } else if (FOLD) {
-            ux += acc.x + (fmaf(Ay, sz, -(Az * sy)) - Bx);
-            uy += acc.y + (fmaf(Az, sx, -(Ax * sz)) - By);
-            uz += acc.z + (fmaf(Ax, sy, -(Ay * sx)) - Bz);
+            ux += acc.x + nx;
+            uy += acc.y + ny;
+            uz += acc.z + nz;
         } else {
             const float k = P->inv4pia3_f;
-            ux = fmaf(acc.x + (fmaf(Ay, sz, -(Az * sy)) - Bx), k, ux);
-            uy = fmaf(acc.y + (fmaf(Az, sx, -(Ax * sz)) - By), k, uy);
-            uz = fmaf(acc.z + (fmaf(Ax, sy, -(Ay * sx)) - Bz), k, uz);
+            ux = fmaf(acc.x + nx, k, ux);
+            uy = fmaf(acc.y + ny, k, uy);
+            uz = fmaf(acc.z + nz, k, uz);
         }
         if (P->status != 0) {
             // zero or non-finite domain edge (one vortex, or all coincident):

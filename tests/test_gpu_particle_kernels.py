@@ -101,6 +101,40 @@ def test_evaluation_from_sparse_to_dense(pb, oracle, per_cell, seg):
     assert rel_l2(u[sub], ref) <= 1e-5
 
 
+@pytest.mark.parametrize("a_cells", [0.0, 1.0])
+@pytest.mark.parametrize("seg", [0, 1])
+@pytest.mark.parametrize("M", [1000, 270000])
+def test_points_without_a_near_field_leave_the_others_alone(pb, oracle, M, seg, a_cells):
+    """Points at infinity, far outside the grid or not a number, which the
+    evaluation order puts next to points at the grid's faces (a block's warps
+    sharing a walk and not): those have their values, a point outside has
+    none.  Far-field interpolation as everywhere, hence the same 1e-5."""
+    rng = np.random.default_rng(M + seg)
+    n, N = 16, 20000
+    pos, al = _points(rng, N), rng.normal(size=(N, 3))
+    ev = _points(rng, M, 0.001, 0.999)
+    odd = np.arange(M) % 20
+    bad = odd < 5
+    ev[odd == 0, 0] = np.inf
+    ev[odd == 1, 1] = -np.inf
+    ev[odd == 2, :3] = 1e30
+    ev[odd == 3, 2] = np.nan
+    ev[odd == 4, 0] += 3.0
+    other = ev.copy()
+    other[:, 1] += np.float32(0.2 / n)
+    scene = pb.Scene(n, K=1, a=0.3, a_cells=a_cells, cap_vort=N, cap_eval=M, domain="fixed", **BOX)
+    scene.set_vortices(_dev(pos), _dev(al.T))
+    scene.build_far_field()
+    u = scene.eval(_dev(ev), _dev(other), seg).cpu().numpy()
+    a = scene.smoothing()
+    scene.close()
+    sub = np.flatnonzero(~bad)[:1000]
+    ref = oracle.pppm(oracle.params(n, K=1, a=a, domain_mode=1, **BOX), pos, al, ev[sub], other[sub], seg)[0]
+    assert rel_l2(u[sub], ref) <= 1e-5
+    assert np.isfinite(u[~bad]).all()
+    assert (u[bad & (odd != 3)] == 0.0).all()
+
+
 def test_deposit_of_uneven_cells(pb, oracle):
     """Rows of cells with none, one and hundreds of vortices, and vortices on
     cell faces (whose nearest cell may not be their hash cell)."""
