@@ -210,7 +210,7 @@ extern "C" pppm_status pppm_batch_run(pppm_batch_item *items, uint32_t count, vo
     for (uint32_t i = 0; i < count; i++)
         if (has_eval[i]) {
             ev.push_back(i);
-            nwork += pppm::eval_blocks(items[i].M);
+            nwork += pppm::eval_blocks(args[i].K, args[i].M);
         }
     std::stable_sort(ev.begin(), ev.end(),
                      [&](uint32_t a, uint32_t b) { return pairs_per_point(items[a]) > pairs_per_point(items[b]); });
@@ -228,7 +228,7 @@ extern "C" pppm_status pppm_batch_run(pppm_batch_item *items, uint32_t count, vo
             if (done[i] || !modes[i].same(modes[lead])) continue;
             done[i] = 1;
             set->args_h[a_pos] = args[i];
-            const uint32_t blocks = pppm::eval_blocks(items[i].M);
+            const uint32_t blocks = pppm::eval_blocks(args[i].K, args[i].M);
             for (uint32_t b = 0; b < blocks; b++) set->work_h[wpos++] = make_uint2(a_pos - a_first, b);
             a_pos++;
         }

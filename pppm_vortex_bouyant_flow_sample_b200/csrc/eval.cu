@@ -1000,11 +1000,13 @@ static EvalArgs make_args(pppm_scene *s, const float4 *eval_a, const float4 *eva
 // their walk: with fewer than about two warps of points for each that the GPU
 // holds, the longest walks (the densest part of a scene) set the time, and a
 // quarter of a walk is what each warp then does (65,537 points, K = 3: 5.6 ms
-// without, 2.6 ms with it).
+// without, 2.6 ms with it).  Without a near field (K < 0) there is no walk to
+// share: the interpolation of 200,000 points took 21 us with three idle warps in
+// each block, 17 us in whole blocks.
 constexpr uint32_t kSplitMaxPoints = 2 * 148 * kEvalBlocksPerSM * kEvalThreads;
-static bool eval_split(uint32_t M) { return M <= kSplitMaxPoints; }
-uint32_t eval_blocks(uint32_t M) {
-    const uint32_t per = eval_split(M) ? 32 : kEvalThreads;
+static bool eval_split(int K, uint32_t M) { return K >= 0 && M <= kSplitMaxPoints; }
+uint32_t eval_blocks(int K, uint32_t M) {
+    const uint32_t per = eval_split(K, M) ? 32 : kEvalThreads;
     return (M + per - 1) / per;
 }
 
@@ -1021,8 +1023,8 @@ cudaError_t launch_eval(pppm_scene *s, const float4 *eval_a, const float4 *eval_
     prof_begin(s, kStageEval);
     ::pppm::note_launch();
     const bool seg = (is_segment == 1) && (eval_b != eval_a);
-    const bool split = eval_split(M);
-    const unsigned grid = eval_blocks(M);
+    const bool split = eval_split(s->prm.K, M);
+    const unsigned grid = eval_blocks(s->prm.K, M);
     SmoothSeries sc;
     const bool fold = make_series(s, sc);
     const EvalArgs ea = make_args(s, eval_a, eval_b, M, u, v, w, uf, count_pairs ? s->pair_count : nullptr);
@@ -1051,7 +1053,7 @@ cudaError_t eval_batch_prepare(pppm_scene *s, const float4 *eval_a, const float4
     static_assert(sizeof(SmoothSeries) <= sizeof(mode->series), "series bytes");
     memcpy(mode->series, &sc, sizeof(sc));
     mode->seg = (is_segment == 1) && (eval_b != eval_a);
-    mode->split = eval_split(M);
+    mode->split = eval_split(s->prm.K, M);
     *args = make_args(s, eval_a, eval_b, M, u, v, w, nullptr, nullptr);
     return cudaSuccess;
 }

@@ -311,7 +311,7 @@ struct EvalMode {
 };
 cudaError_t eval_batch_prepare(pppm_scene *s, const float4 *eval_a, const float4 *eval_b, int is_segment, uint32_t M,
                                double *u, double *v, double *w, EvalArgs *args, EvalMode *mode);
-uint32_t eval_blocks(uint32_t M);  // blocks of the evaluation of M points
+uint32_t eval_blocks(int K, uint32_t M);  // blocks of the evaluation of M points
 cudaError_t launch_eval_batch(const EvalMode &mode, const EvalArgs *args_dev, const uint2 *work_dev, uint32_t blocks,
                               cudaStream_t st);
 cudaError_t launch_gather_sorted(pppm_scene *s, float4 *pos_out, double *alpha_out);

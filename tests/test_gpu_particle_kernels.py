@@ -77,6 +77,29 @@ def test_evaluation_of_few_points(pb, oracle, M, a_cells, K):
     assert rel_l2(u, ref) <= 1e-5
 
 
+@pytest.mark.parametrize("M", [1, 32, 33, 127, 128, 129, 700])
+def test_far_field_only_evaluation(pb, oracle, M):
+    """K = -1 takes whole blocks of points at every size, alone and in a batch
+    beside a scene with a near field (32 points a block)."""
+    rng = np.random.default_rng(M)
+    n, N = 16, 3000
+    pos, al, ev = _points(rng, N), rng.normal(size=(N, 3)), _points(rng, M, -0.05, 1.05)
+    jobs, want = [], []
+    for K in (-1, 1):
+        scene = pb.Scene(n, K=K, a=0.3, cap_vort=N, cap_eval=M, domain="fixed", **BOX)
+        jobs.append((scene, _dev(pos), _dev(al.T), _dev(ev), None, 0))
+        want.append(oracle.pppm(oracle.params(n, K=K, a=0.3, domain_mode=1, **BOX), pos, al, ev, None, 0)[0])
+    batch = [u.cpu().numpy() for u in pb.batch_run(jobs)]
+    scene = jobs[0][0]
+    scene.set_vortices(*jobs[0][1:3])
+    scene.build_far_field()
+    alone = scene.eval(jobs[0][3]).cpu().numpy()
+    for got, ref in ((alone, want[0]), (batch[0], want[0]), (batch[1], want[1])):
+        assert rel_l2(got, ref) <= 1e-5
+    for j in jobs:
+        j[0].close()
+
+
 @pytest.mark.parametrize("per_cell", [0.3, 2.0, 6.0, 20.0])
 @pytest.mark.parametrize("seg", [0, 1])
 def test_evaluation_from_sparse_to_dense(pb, oracle, per_cell, seg):
