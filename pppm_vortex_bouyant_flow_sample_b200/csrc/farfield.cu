@@ -299,7 +299,13 @@ cudaError_t launch_farfield(pppm_scene *s) {
     const unsigned blocks = (s->C + kFFThreads - 1) / kFFThreads;
     ::pppm::note_launch();
     const int n = (int)s->n, K = s->prm.K;
-    if (K >= 0 && n % 4 == 0) {
+    // K = 0 reads no neighbours beside the two curls', so that below edge 48 there
+    // are too few groups of 4 for their longer threads to pay: 2.5 to 3.4 us from
+    // 12^3 to 40^3 with a cell a thread, 2.8 to 3.6 us with four; 3.8 and 3.7 at
+    // 48^3.  With K = 1 four take 8.0, 8.3 and 9.1 us at 8^3, 12^3 and 20^3 where
+    // one takes 8.3, 8.8 and 9.8 (16^3: 8.9 and 8.5), and 12.3 to 13.5 against
+    // 19.3 to 21.2 with K = 2.
+    if (n % 4 == 0 && (K > 0 || (K == 0 && n >= 48))) {
         const int bx = std::min(32, n / 4);
         const dim3 block(bx, kFFThreads / bx), grid((n / 4 + block.x - 1) / block.x, (n + block.y - 1) / block.y, n);
         auto *f = K == 0 ? farfield4_kernel<0>

@@ -91,12 +91,13 @@ def test_corrected_cycles_reach_the_tolerance(pb, oracle, n, tol):
     assert abs(rel - got) <= 1e-6 * got + 1e-14
 
 
-@pytest.mark.parametrize("K", [-1, 0, 1, 2, 4])
-@pytest.mark.parametrize("n", [10, 12, 20])
+@pytest.mark.parametrize("n,K", [(n, K) for n in (10, 12, 20) for K in (-1, 0, 1, 2, 4)] +
+                         [(40, 0), (48, 0), (160, 1), (160, 2)])
 def test_far_field_grid(pb, oracle, n, K):
     """The far-field grid of the four-cell kernel (edges that are multiples of
-    4: rows of 3 and 5 groups, windows beyond both ends) and of the one-cell
-    kernel (10): FP32 sums of at most 728 terms beside an FP64 curl, so 1e-5."""
+    4, from 48 with K = 0: rows of 3 and 5 groups, windows beyond both ends, and
+    of 40, which two blocks share) and of the one-cell kernel: FP32 sums of at
+    most 728 terms beside an FP64 curl, so 1e-5."""
     import torch
     rng = np.random.default_rng(5)
     N = 900
