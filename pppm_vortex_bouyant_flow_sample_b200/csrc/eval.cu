@@ -19,15 +19,16 @@
 //     which equals (1 - e^-(r/a)^3) / (4 pi r^3); pairs with r = 0, or (for
 //     segments) a zero distance to the other end, are skipped.
 // Pair arithmetic is FP32 (r^3 = r^2 sqrt.approx(r^2) in the warp-uniform walk,
-// r^2 rsqrt(r^2) in a lane's own walk; ~1 ulp).  phi: when no pair of the
-// scene can reach t = 0.25, a degree-4 polynomial (Chebyshev interpolant on
-// [0, 0.25], relative error 5e-9); otherwise a degree-7 one on [0, 2] (relative
-// error 2e-7, below that of the exp form near t = 0.25) and (1 - exp(-t)) / t
-// above t = 2.  No cancellation in either polynomial.  When some pair can
-// reach t = 2 (a smoothing radius of about a cell or less), the warp-uniform
-// walk takes the exp form (1 - e^-t) / (4 pi r^3) for every pair, r^-1 from
-// rsqrt.approx and e^-t from ex2.approx, with a degree-5 polynomial of phi
-// below t = 1/64, where 1 - e^-t would cancel.
+// r^2 rsqrt(r^2) in a lane's own walk; ~1 ulp).  phi in the warp-uniform walk:
+// when no pair of the scene can reach t = 0.25, a degree-4 polynomial (Chebyshev
+// interpolant on [0, 0.25], relative error 5e-9); when none can reach t = 2, a
+// degree-7 one on [0, 2] (relative error 2e-7, below that of the exp form near
+// t = 0.25).  No cancellation in either polynomial.  When some pair can reach
+// t = 2 (a smoothing radius of about a cell or less), the exp form
+// (1 - e^-t) / (4 pi r^3) for every pair, r^-1 from rsqrt.approx and e^-t from
+// ex2.approx, with a degree-5 polynomial of phi below t = 1/64, where 1 - e^-t
+// would cancel.  A lane's own walk takes the degree-4 polynomial below t = 0.25
+// and (1 - exp(-t)) / t above.
 #include <climits>
 #include <cstring>
 #include <cmath>
@@ -111,11 +112,8 @@ struct PairAcc {
 // phi(t) = (1 - e^-t) / t, scaled by 1/(4 pi a^3).  Below t = 0.25 a degree-4
 // polynomial (the interpolant at the 5 Chebyshev nodes of [0, 0.25], relative
 // error below 5e-9 with float coefficients) needs no special function; its
-// coefficients arrive pre-scaled by 1/(4 pi a^3) in cf[0..4].  Above t = 0.25,
-// (1 - exp(-t)) / t.  The exp branch runs only when the scene can reach it
-// and some lane of the warp needs it (UNIFORM: the whole warp executes this
-// call together; otherwise each lane branches on its own t).
-template <bool UNIFORM>
+// coefficients arrive pre-scaled by 1/(4 pi a^3) in cf[0..4].  Above it
+// (1 - exp(-t)) / t, where the scene can get there (need_exp).
 __device__ __forceinline__ float smooth_coeff(float t, const float *cf, float inv4pia3, bool need_exp) {
     float p = cf[4];
     p = fmaf(p, t, cf[3]);
@@ -123,11 +121,7 @@ __device__ __forceinline__ float smooth_coeff(float t, const float *cf, float in
     p = fmaf(p, t, cf[1]);
     p = fmaf(p, t, cf[0]);
     if (need_exp) {
-        const bool big = t >= 0.25f;
-        if (UNIFORM ? __any_sync(0xffffffffu, big) : big) {
-            const float e = __fdividef(1.0f - __expf(-t), fmaxf(t, 0.25f)) * inv4pia3;
-            p = big ? e : p;
-        }
+        if (t >= 0.25f) p = __fdividef(1.0f - __expf(-t), t) * inv4pia3;
     }
     return p;
 }
@@ -135,7 +129,7 @@ __device__ __forceinline__ float smooth_coeff(float t, const float *cf, float in
 // One candidate pair, branch free: the box test, the lane's cell range and
 // the zero-distance exclusions become a zero coefficient.  SEG: test the
 // segment's other end; COUNT: count the pairs inside the box.
-template <bool SEG, bool COUNT, bool UNIFORM>
+template <bool SEG, bool COUNT>
 __device__ __forceinline__ void pair_term(const float4 r, const float4 al, bool lane_ok, const float3 ra,
                                           const float3 rb, float cr, float inv_a3, const float *cf, float inv4pia3,
                                           bool need_exp, PairAcc &acc) {
@@ -150,7 +144,7 @@ __device__ __forceinline__ void pair_term(const float4 r, const float4 al, bool 
         ok = ok && !(fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < 1e-24f);
     }
     const float rr = r2 * rsqrtf(fmaxf(r2, 1e-30f));
-    const float c = smooth_coeff<UNIFORM>(r2 * rr * inv_a3, cf, inv4pia3, need_exp);
+    const float c = smooth_coeff(r2 * rr * inv_a3, cf, inv4pia3, need_exp);
     const float coeff = ok ? c : 0.0f;
     acc.x = fmaf(al.y * dz - al.z * dy, coeff, acc.x);
     acc.y = fmaf(al.z * dx - al.x * dz, coeff, acc.y);
@@ -164,7 +158,7 @@ __device__ __forceinline__ void cell_pairs(const float4 *__restrict__ vrec, cons
                                            float cr, float inv_a3, const float *cf, float inv4pia3, bool need_exp,
                                            PairAcc &acc) {
     for (uint32_t p = ps; p < pe; p++)
-        pair_term<SEG, COUNT, false>(vrec[p], valf[p], lane_ok, ra, rb, cr, inv_a3, cf, inv4pia3, need_exp, acc);
+        pair_term<SEG, COUNT>(vrec[p], valf[p], lane_ok, ra, rb, cr, inv_a3, cf, inv4pia3, need_exp, acc);
 }
 
 // The near-field sum of a target,
@@ -290,13 +284,12 @@ __device__ __forceinline__ float2 exp_coeff(float2 dx, float2 dy, float2 dz, con
     return c;
 }
 
-// phi of two pairs at (dx, dy, dz): the degree-DEG polynomial cf (DEG 4: the
-// scene never leaves [0, 0.25]; DEG 7: valid on [0, 2], the exp form above tbig
-// when need_exp), or (DEG 0) the exp form.  FOLD: the coefficients carry the
-// powers of 1/a^3, so the polynomial takes r^3 directly and tbig is in r^3 too.
+// phi of two pairs at (dx, dy, dz): the degree-DEG polynomial cf (DEG 4 for
+// scenes that never leave [0, 0.25], DEG 7 for those that stay below t = 2), or
+// (DEG 0) the exp form.  FOLD: the coefficients carry the powers of 1/a^3, so
+// the polynomial takes r^3 directly.
 template <bool FOLD, int DEG, bool CHECK>
-__device__ __forceinline__ float2 phi_coeff(float2 dx, float2 dy, float2 dz, bool ok0, bool ok1, float2 inv_a3,
-                                            const float2 *cf, float tbig, float inv4pia3, bool need_exp,
+__device__ __forceinline__ float2 phi_coeff(float2 dx, float2 dy, float2 dz, float2 inv_a3, const float2 *cf,
                                             const ExpForm &xf) {
     float2 c;
     if constexpr (DEG == 0) {
@@ -308,16 +301,6 @@ __device__ __forceinline__ float2 phi_coeff(float2 dx, float2 dy, float2 dz, boo
         c = __ffma2_rn(cf[DEG], t3, cf[DEG - 1]);
 #pragma unroll
         for (int q = DEG - 2; q >= 0; q--) c = __ffma2_rn(c, t3, cf[q]);
-        if (DEG > 4 && need_exp) {
-            const bool big0 = ok0 && t3.x >= tbig, big1 = ok1 && t3.y >= tbig;
-            if (__any_sync(0xffffffffu, big0 || big1)) {
-                const float v0 = FOLD ? t3.x * inv_a3.x : t3.x, v1 = FOLD ? t3.y * inv_a3.y : t3.y;
-                const float e0 = __fdividef(1.0f - __expf(-v0), fmaxf(v0, 1.0f)) * inv4pia3;
-                const float e1 = __fdividef(1.0f - __expf(-v1), fmaxf(v1, 1.0f)) * inv4pia3;
-                c.x = big0 ? e0 : c.x;
-                c.y = big1 ? e1 : c.y;
-            }
-        }
     }
     return c;
 }
@@ -350,8 +333,7 @@ __device__ __forceinline__ void stage_record(WarpMem &W, uint32_t e, float4 r, f
 template <int OTHER, bool COUNT, bool FOLD, int DEG, bool FULL, bool CHECK>
 __device__ __forceinline__ void pair_block(const WarpMem &W, uint32_t s0, uint32_t np, float cr_lane,
                                              const float3 ra, const float3 rb, uint32_t pstar, float2 inv_a3,
-                                             const float2 *cf, float tbig, float inv4pia3, bool need_exp,
-                                             const ExpForm &xf, PairSums &acc) {
+                                             const float2 *cf, const ExpForm &xf, PairSums &acc) {
     const float2 tx = make_float2(ra.x, ra.x), ty = make_float2(ra.y, ra.y), tz = make_float2(ra.z, ra.z);
     const uint32_t cnt = FULL ? kBlockRecs / 2 : np;
 #pragma unroll (FULL ? kBlockRecs / 2 : 2)
@@ -375,7 +357,7 @@ __device__ __forceinline__ void pair_block(const WarpMem &W, uint32_t s0, uint32
             ok0 = ok0 && !(e2.x < 1e-24f);
             ok1 = ok1 && !(e2.y < 1e-24f);
         }
-        const float2 c = phi_coeff<FOLD, DEG, CHECK>(dx, dy, dz, ok0, ok1, inv_a3, cf, tbig, inv4pia3, need_exp, xf);
+        const float2 c = phi_coeff<FOLD, DEG, CHECK>(dx, dy, dz, inv_a3, cf, xf);
         // the exp form's c is finite for every pair of a lane with a point (r = 0
         // takes the polynomial), so the box mask can multiply it; the polynomials
         // can overflow on the padding record
@@ -413,7 +395,6 @@ struct SmoothSeries {
     float2 p4[5];  // degree 4 on [0, 0.25], packed
     float2 p7[8];  // degree 7 on [0, 2], packed
     float2 p5[6];  // degree 5 on [0, 0.5] in t, unit scale (exp-form walk)
-    float t7;      // 2 in the packed polynomials' variable: where the exp form takes over
 };
 
 // One block of evaluation points of one scene: kEvalThreads consecutive points
@@ -466,7 +447,6 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
         const float *cf = sc.c;
         // some pair can reach t = 0.25 (but not 2): the degree-7 polynomial
         const bool tier7 = need_exp && !tier0;
-        const bool need_exp2 = P->need_exp2 != 0;
         ExpForm xf;
         xf.inv_a3 = make_float2(inv_a3, inv_a3);
         xf.nl2a3 = make_float2(-1.4426950408889634f * inv_a3, -1.4426950408889634f * inv_a3);
@@ -616,7 +596,7 @@ __device__ __forceinline__ void eval_points(const SmoothSeries &sc, const EvalAr
             auto block = [&](auto full, auto check, uint32_t s0, uint32_t recs) {
                 constexpr bool FULL = decltype(full)::value, CHECK = decltype(check)::value;
                 pair_block<S, COUNT, FOLD, D, FULL, CHECK>(W, s0, recs >> 1, (COUNT ? box : act) ? cr : -1.0f, ra, rb, pstar, inv_a3_2,
-                                                           cfd, sc.t7, inv4pia3, D == 7 && need_exp2, xf, sums);
+                                                           cfd, xf, sums);
             };
             // The runs of records, one per (cell, y and z halves): the two x
             // halves of a cell are adjacent.  The lanes look up 32 runs at
@@ -968,7 +948,6 @@ static bool make_series(const pppm_scene *s, SmoothSeries &sc) {
         const float v7 = fold ? (float)u7[q] : (float)(k * f7[q]);
         sc.p7[q] = make_float2(v7, v7);
     }
-    sc.t7 = fold ? (float)(2.0 * s->prm.a * s->prm.a * s->prm.a) : 2.0f;
     return fold;
 }
 
