@@ -54,7 +54,7 @@ def test_sort_is_stable_at_every_size(pb, n, N):
     assert np.array_equal(key, want[order])
 
 
-@pytest.mark.parametrize("K", [0, 1, 3])
+@pytest.mark.parametrize("K", [0, 1, 3, 4])
 @pytest.mark.parametrize("a_cells", [0.0, 1.0])
 @pytest.mark.parametrize("M", [1, 15, 16, 17, 32, 33, 129, 700])
 def test_evaluation_of_few_points(pb, oracle, M, a_cells, K):
