@@ -66,7 +66,7 @@ def workload(N: int, n: int, preset: str = "configured") -> str:
     what = {"configured": "K=1, a=1 cell", "reference_constants": "K=1, a=0.08 (the reference's constant)",
             "accurate": "K=3, a=1 cell, multigrid to 1e-6 (accurate preset)"}[preset]
     mg = ("FMG + 1 V(4,4), FP32 with FP64 defect correction" if preset != "accurate"
-          else "FMG + FP64 defect-correction V(4,4) cycles to 1e-6")
+          else "FP64 defect-correction V(2,2) cycles to 1e-6")
     return (f"vortex ring, {N:,} particles, {n}^3 grid, {what}, domain 3x bbox, {mg}; "
             "step = far-field build + velocity at every particle")
 

@@ -52,8 +52,14 @@ enum { PPPM_DOMAIN_BBOX3X = 0, PPPM_DOMAIN_FIXED = 1 };
  * one V(4,4) cycle, red-black SOR with omega = 1.43f, zero ghost values, 100
  * Jacobi sweeps on the coarsest level (MG/MultiGrid.cpp:128-250) — in FP32,
  * with the final V-cycle applied as an FP64 defect correction (FP64
- * residual, FP64 accumulation of psi).  CONVERGED repeats FP64
- * defect-correction V-cycles until ||b - A psi|| <= mg_tol * ||b||. */
+ * residual, FP64 accumulation of psi).  CONVERGED chooses its own cycles, each
+ * an FP64 defect correction: V(2,2) with omega = 1.25f, the coarse levels'
+ * zero ghost values moved to where the finest level has them, and trilinear
+ * prolongation (a grid of at most 512 cells repeats its coarsest solve).  It
+ * stops at ||b - A psi|| <= mg_tol * ||b|| or after mg_max_cycles.  The first
+ * two cycles, which stand for the full multigrid and its V-cycle, count as one;
+ * a residual between 0.2 mg_tol and mg_tol gets one cycle more, if the cap
+ * allows it. */
 enum { PPPM_MG_REFERENCE = 0, PPPM_MG_CONVERGED = 1 };
 
 typedef struct pppm_params {
@@ -66,7 +72,7 @@ typedef struct pppm_params {
     double fixed_length;
     int32_t mg_mode;         /* PPPM_MG_*                                         */
     double mg_tol;           /* relative residual target for CONVERGED            */
-    int32_t mg_max_cycles;   /* cap on defect-correction cycles                   */
+    int32_t mg_max_cycles;   /* cap on the cycles of CONVERGED as they are counted */
     double a_cells;          /* > 0: smoothing radius in cells, a = a_cells * h with
                                 h the cell size of each build's domain (overrides a);
                                 0: a is absolute, as in the reference              */
@@ -221,7 +227,8 @@ pppm_status pppm_get_sorted_vortices(pppm_scene *s, float *pos4_dev, double *ax_
                                      double *ay_dev, double *az_dev);
 pppm_status pppm_get_grid(pppm_scene *s, int which, const void **ptr_dev);
 /* Near-field pairs inside the axis box at the last eval with pair counting
- * on, multigrid cycles and final relative residual of the last solve. */
+ * on, multigrid cycles (as mg_max_cycles counts them) and final relative
+ * residual of the last solve. */
 pppm_status pppm_get_stats(pppm_scene *s, uint64_t *pairs, int32_t *mg_cycles,
                            double *mg_relres);
 /* Re-runs the last eval with pair counting on (diagnostics; not timed). */
@@ -368,9 +375,9 @@ pppm_status pppm_mg_destroy(pppm_mg *mg);
  * sum_nbr(x) - 6x = b with zero ghost values, starting from the x given (the
  * reference's first residual is b - A x): x <- x + FMG(0, b - A x).
  * mode = PPPM_MG_REFERENCE runs the reference schedule (tol ignored, as in the
- * reference); CONVERGED adds defect-correction cycles until the residual is
- * below tol relative to ||b - A x_initial||, which *relres (may be NULL)
- * receives. */
+ * reference); CONVERGED takes its own cycles, counted as for a scene, until the
+ * residual is below tol relative to ||b - A x_initial||; *relres (may be NULL)
+ * receives that ratio.  x and b need only be aligned as doubles. */
 pppm_status pppm_mg_full_multigrid(pppm_mg *mg, double *x_dev, const double *b_dev,
                                    int mode, double tol, int max_cycles, double *relres);
 /* m_Vcycle(x, b, tol, residual, level) (MG/MultiGrid.cpp:128-201): one V(4,4)
@@ -378,7 +385,8 @@ pppm_status pppm_mg_full_multigrid(pppm_mg *mg, double *x_dev, const double *b_d
  * arrays x and b of d_level^3 entries (level 0 = the n^3 grid).  Applied as a
  * defect correction: r = b - A x in FP64, an FP32 cycle on A e = r from
  * e = 0, x += e in FP64 — the reference's cycle in exact arithmetic.  The
- * reference ignores tol and leaves residual unset; so does the C++ mirror. */
+ * reference ignores tol and leaves residual unset; so does the C++ mirror.  x
+ * and b need only be aligned as doubles. */
 pppm_status pppm_mg_vcycle(pppm_mg *mg, double *x_dev, const double *b_dev, int level);
 /* Level count of the hierarchy (halve while a level has more than 512 cells,
  * MG/MultiGrid.h:114-127) and the edge of each level (up to cap entries). */
@@ -474,7 +482,8 @@ pppm_status pppm_hasher_deorder(pppm_hasher *h, uint32_t N, const void *in_dev, 
  *     address is stale: do not call this entry point again in that process.
  *   - All calls share the array: calls whose work overlaps on the GPU (other
  *     streams, other threads) race and corrupt each other's results.
- *   - No cudaMalloc, cudaFree or allocating library routine is called. */
+ *   - No cudaMalloc, cudaFree or allocating library routine is called.
+ *   - The output arrays need only be aligned as uint32_t. */
 #define PPPM_NOALLOC_MAX_PARTICLES 1048576u
 #define PPPM_NOALLOC_SCRATCH_BYTES 8651776u
 pppm_status pppm_spatial_hash_noalloc(uint32_t N, const float *pos4_dev, uint32_t n, float cell_h,

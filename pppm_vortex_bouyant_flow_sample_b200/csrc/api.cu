@@ -142,7 +142,7 @@ cudaError_t alloc_vortex_buffers(pppm_scene *s, uint32_t cap) {
     PPPM_CUDA_TRY(dalloc(&s->valf, cap));
     PPPM_CUDA_TRY(dalloc(&s->adv_mid, cap));
     PPPM_CUDA_TRY(dalloc(&s->ts_kappa, cap));
-    s->bbox_blocks = 148 * 2;
+    s->bbox_blocks = 2 * pppm::kSMs;
     PPPM_CUDA_TRY(dalloc(&s->bbox_partial, 6 * (size_t)s->bbox_blocks));
     return cudaSuccess;
 }
@@ -958,7 +958,7 @@ extern "C" pppm_status pppm_mg_create(uint32_t n, void *stream, pppm_mg **out) {
             cudaFree(m->r64);
             cudaFree(m->e64);
             cudaFree(m->scratch);
-                cudaFree(m->x2_pool);
+            cudaFree(m->x2_pool);
             cudaFree(m->err);
             delete m;
             return st;

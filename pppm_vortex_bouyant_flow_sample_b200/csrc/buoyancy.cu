@@ -377,7 +377,7 @@ extern "C" pppm_status pppm_baroclinic(pppm_scene *s, uint32_t H, const float *h
     const float of[3] = {(float)origin[0], (float)origin[1], (float)origin[2]};
     const uint32_t cells = dim * dim * dim;
     // slices per cell: enough warps to fill the GPU when the grid is small
-    uint32_t S = (uint32_t)std::min<uint64_t>(kMaxSplit, std::max<uint64_t>(1, (148ull * 32) / cells));
+    uint32_t S = (uint32_t)std::min<uint64_t>(kMaxSplit, std::max<uint64_t>(1, (32ull * kSMs) / cells));
     e = ensure_grid(b, cells, S > 1 ? (size_t)cells * S : 0);
     if (e != cudaSuccess) {
         pppm_set_error("pppm_baroclinic (grid alloc): %s", cudaGetErrorString(e));

@@ -990,7 +990,7 @@ static EvalArgs make_args(pppm_scene *s, const float4 *eval_a, const float4 *eva
 // without, 2.6 ms with it).  Without a near field (K < 0) there is no walk to
 // share: the interpolation of 200,000 points took 21 us with three idle warps in
 // each block, 17 us in whole blocks.
-constexpr uint32_t kSplitMaxPoints = 2 * 148 * kEvalBlocksPerSM * kEvalThreads;
+constexpr uint32_t kSplitMaxPoints = 2 * kSMs * kEvalBlocksPerSM * kEvalThreads;
 static bool eval_split(int K, uint32_t M) { return K >= 0 && M <= kSplitMaxPoints; }
 uint32_t eval_blocks(int K, uint32_t M) {
     const uint32_t per = eval_split(K, M) ? 32 : kEvalThreads;

@@ -114,9 +114,9 @@ farfield_kernel(const double *__restrict__ psi, const float *__restrict__ vort, 
 // of its (2K+1)^2 neighbour rows once with 128-bit loads, 4 + 2K values that
 // serve its 4 cells, instead of 2K+1 scalars a cell, and each table entry once;
 // the one-cell kernel issues 81 loads and 26 table reads a cell at K = 1 and is
-// bound by them.  K = 1 on B200: 1206 to 470 us at 256^3 (its 72 bytes a cell
-// take 185 us at the copy rate), 156 to 60 us at 128^3; at 16^3, where a launch
-// is all there is, 7.7 to 9.2 us.
+// bound by them.  K = 1 on B200: 1206 to 437 us at 256^3 (its 48 bytes a cell
+// take 123 us at the copy rate), 156 to 57 us at 128^3; small grids: see
+// launch_farfield.
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 
 __device__ __forceinline__ void load_row(const double *__restrict__ row, double *v) {

@@ -317,8 +317,8 @@ __device__ __forceinline__ void warp_ranks(const uint32_t (&k)[kItems], int shif
 // digit's run is then written by consecutive threads.  With a block barrier for
 // each round of 256 keys and the keys written where they fell, a pass over 1M
 // keys took 14 us; so it takes 9 (16 MB: 2.5 us at the copy rate; the ranks'
-// serial rounds are the rest).  The counts before it, with 128-bit loads and
-// a warp's own counters: 6.4 to 3.0 us.
+// serial rounds are the rest).  The counts before it, with 128-bit loads: 6.4 to
+// 3.0 us.
 __global__ void __launch_bounds__(kRsThreads)
 radix_downsweep_kernel(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
                        uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, uint32_t N, int shift,

@@ -1,9 +1,9 @@
 // A whole red-black sweep (both half sweeps) of a level in one pass over it.
 //
-// A half sweep by itself streams x and b once and x back, 12 B a cell, so a
-// sweep of two moves 24 B a cell: 1.2 GB at 256^3 with three components, which
-// is what bounds the smoother there, and at 64^3 and 128^3 (in L2) two
-// launches.  This kernel reads x and b once and writes x once for the two.
+// A pass over one colour streams x and b once and x back, 12 B a cell, so a
+// sweep of two would move 24 B a cell, 1.2 GB at 256^3 with three components
+// (HBM bounds the smoother there), and be two launches where the level lies in
+// L2 (64^3, 128^3).  This kernel reads x and b once and writes x once for both.
 //
 // A CTA owns TY whole rows (in y) and a chunk of planes, and walks the chunk
 // upwards.  A thread holds a group of 4 consecutive cells of two rows, for
@@ -17,16 +17,19 @@
 // memory it has just asked for.  Which cells have the colour depends on z and
 // the thread's row only, so the steps come in two kinds without a select.
 // Measured on B200, three components: 106 us a sweep at 256^3 and 14.6 us at
-// 128^3, against 188 us and 26.4 us for two one-colour passes.  The 30 sweeps
-// (128^3 and 64^3) of a 128^3 solve take 316 us; with the loads in registers
-// one step ahead they took 396 us, with a select per cell 332 us.
+// 128^3, against 188 us and 26.4 us for two passes of one colour each.  A 128^3
+// solve holds 40 sweeps, 16 of them at 128^3 and 24 at 64^3.  The 30 that read x
+// and add no correction take 314 us; with the loads in registers one step ahead
+// they took 396 us, with a select per cell 332 us.  At 64^3 a sweep takes 4.4 to
+// 5.7 us for about 1 us of data: its chunks are no thinner than 4 planes, each
+// walks 4 more, and few blocks run.
 // The rows and planes next to a CTA's own are updated by it too (the first
 // colour: one row or plane each side, from values two away), which costs 4
 // extra rows and 4 extra planes of reads but no exchange.  Since neighbours
 // still read the old values, the result goes to the level's second copy of x.
 //
-// Each cell gets the terms of the one-colour kernel in its order, so the
-// values are the same bit for bit.
+// Each cell gets the terms of a pass over one colour in the same order, so the
+// values are the same bit for bit (tests compare the blocked smoother's).
 //
 // The start of a smoothing can be folded into the reads: x = 0 (nothing is
 // read or cleared), and the coarser level's correction added.  The end of a
@@ -64,11 +67,6 @@ struct SweepArgs {
 
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 
-// The corrected cycle's update: inv = 1 / diagonal.
-__device__ __forceinline__ float corr_update(float x, float nb, float b, float inv) {
-    return (1.0f - kCorrOmega) * x + kCorrOmega * ((nb - b) * inv);
-}
-
 // The group's 2 cells of a colour: ODD, ODD + 2.
 template <bool CORR, bool ODD>
 __device__ __forceinline__ float4 update_group(float4 v, float xl, float xr, const float4 up, const float4 dn,
@@ -77,13 +75,13 @@ __device__ __forceinline__ float4 update_group(float4 v, float xl, float xr, con
     if (ODD) {
         const float lo = ((v.x + v.z) + (up.y + dn.y)) + (fr.y + bk.y);
         const float hi = ((v.z + xr) + (up.w + dn.w)) + (fr.w + bk.w);
-        v.y = CORR ? corr_update(v.y, lo, bb.y, inv_lo) : mg_sor_update(v.y, lo, bb.y);
-        v.w = CORR ? corr_update(v.w, hi, bb.w, inv_hi) : mg_sor_update(v.w, hi, bb.w);
+        v.y = CORR ? mg_corr_update(v.y, lo, bb.y, inv_lo) : mg_sor_update(v.y, lo, bb.y);
+        v.w = CORR ? mg_corr_update(v.w, hi, bb.w, inv_hi) : mg_sor_update(v.w, hi, bb.w);
     } else {
         const float lo = ((xl + v.y) + (up.x + dn.x)) + (fr.x + bk.x);
         const float hi = ((v.y + v.w) + (up.z + dn.z)) + (fr.z + bk.z);
-        v.x = CORR ? corr_update(v.x, lo, bb.x, inv_lo) : mg_sor_update(v.x, lo, bb.x);
-        v.z = CORR ? corr_update(v.z, hi, bb.z, inv_hi) : mg_sor_update(v.z, hi, bb.z);
+        v.x = CORR ? mg_corr_update(v.x, lo, bb.x, inv_lo) : mg_sor_update(v.x, lo, bb.x);
+        v.z = CORR ? mg_corr_update(v.z, hi, bb.z, inv_hi) : mg_sor_update(v.z, hi, bb.z);
     }
     return v;
 }
@@ -378,7 +376,7 @@ cudaError_t mg_sweep(const SweepSpec &sp, cudaStream_t st) {
     // chunks of planes: fill the resident CTAs in whole waves, each chunk
     // paying 4 planes more than its own
     const int per_sm = std::max(1, std::min({2048 / threads, 65536 / (96 * threads), (int)(227 * 1024 / (smem + 1024))}));
-    const int tiles = (d + a.ty - 1) / a.ty * comps, slots = 148 * per_sm;
+    const int tiles = (d + a.ty - 1) / a.ty * comps, slots = kSMs * per_sm;
     int best = 1;
     long cost = -1;
     for (int c = 1; c <= d / 4; c++) {

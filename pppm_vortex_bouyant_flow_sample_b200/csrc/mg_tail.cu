@@ -18,15 +18,19 @@
 //      at most 8 points, one factor per mode, three transforms back, in FP64.
 //      The reference schedule's 100 Jacobi sweeps from zero are the factor
 //      -(1 - mu^100) / (6 (1 - mu)) with mu the mode's eigenvalue of the
-//      sweep (sine modes); the stored 512 x 512 operator that the one-level
-//      kernels apply would have to be read by one CTA, 2 MB of it.
+//      sweep (sine modes).  Applied as a 512 x 512 matrix the same map would
+//      have one CTA read 2 MB.
 // Edges: the levels halve, every level above the coarsest is even, and the
 // coarsest is the first with at most 512 cells, so a hierarchy has at most
 // one level of each kind; grids of edge 9 to 16 start at B.
 //
-// Sums are taken in the order of the one-level kernels, so A and B hold the
-// same values bit for bit; the coarsest solve agrees with the stored operator
-// to FP64 rounding.
+// Sums are taken in the order of the larger levels' kernels (mg_sweep.cu,
+// mg.cu), so a level holds the same values bit for bit wherever it runs; the
+// coarsest solve agrees with 100 sweeps to FP64 rounding.
+//
+// The basis is formed on the host at each launch: sines, captured once with the
+// graph of the fixed schedule, or, for the corrected cycle, an eigenproblem of at
+// most 8 points that takes 12 us (5 points) to 45 us (8) of host time.
 #include <cooperative_groups.h>
 
 #include <cmath>
@@ -94,14 +98,10 @@ __device__ __forceinline__ float pick4(const float4 &v, int i) {
     return i < 2 ? (i == 0 ? v.x : v.y) : (i == 2 ? v.z : v.w);
 }
 
-__device__ __forceinline__ float corr_update(float x, float nb, float b, float inv) {
-    return (1.0f - kCorrOmega) * x + kCorrOmega * ((nb - b) * inv);
-}
-
 // b restricted to the coarse cell whose first child sits at padded offset o
 // of x and at ob of b: 0.5 * sum of the children's residuals (of b itself
-// when x is zero), in the one-level kernels' order.  CORR: (i, j, k) is the
-// first child, ghost the level's ghost factor.
+// when x is zero), in resid_restrict2_kernel's order (mg.cu).  CORR: (i, j, k)
+// is the first child, ghost the level's ghost factor.
 template <bool CORR>
 __device__ __forceinline__ float restrict8(const float *__restrict__ x, const float *__restrict__ b, int o, int ob,
                                            int d, bool x_zero, float ghost, int i, int j, int k) {
@@ -200,7 +200,7 @@ __device__ __forceinline__ void smooth_b(float *__restrict__ x, const Pair (&it)
                 const int e = (it[q].par + color) & 1;
                 const int o = it[q].off + e;
                 const float nb = nb6(x, o, P), b = e ? bv[q].y : bv[q].x;
-                x[o] = CORR ? corr_update(x[o], nb, b, pick4(inv, e ? it[q].f1 : it[q].f0)) : mg_sor_update(x[o], nb, b);
+                x[o] = CORR ? mg_corr_update(x[o], nb, b, pick4(inv, e ? it[q].f1 : it[q].f0)) : mg_sor_update(x[o], nb, b);
             }
         }
         __syncthreads();
@@ -385,7 +385,7 @@ mg_tail_kernel(const TailArgs a) {
                     const int e = (ita[q].par + color) & 1;
                     const int o = ita[q].off + e;
                     const float nb = nb6(S.xa, o, PA), b = e ? bva[q].y : bva[q].x;
-                    const float v = CORR ? corr_update(S.xa[o], nb, b, pick4(a.invA, e ? ita[q].f1 : ita[q].f0))
+                    const float v = CORR ? mg_corr_update(S.xa[o], nb, b, pick4(a.invA, e ? ita[q].f1 : ita[q].f0))
                                          : mg_sor_update(S.xa[o], nb, b);
                     S.xa[o] = v;
                     if (ita[q].first) down[o] = v;

@@ -24,6 +24,7 @@ namespace pppm {
 
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 constexpr int kMaxLevels = 12;
+constexpr int kSMs = 148;  // of a B200
 constexpr int kMaxK = 4;  // near-field range limit (table (2K+1)^3 in shared memory)
 constexpr uint32_t kRsTileHost = 4096;  // radix-sort keys per block (kRsThreads * kRsItems)
 
@@ -88,7 +89,7 @@ struct MGPlan {
     // maps and z-chunk length (levels with edge >= tb_min_edge, x2 allocated),
     // and the device error flag
     int tb_var[kMaxLevels] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1};
-    uint32_t tb_min_edge = 256;  // smaller levels measured faster with one-colour passes
+    uint32_t tb_min_edge = 256;  // below it the sweep kernel runs alone
     bool tb_fuse_prolong = false;  // prolongation inside the first post-smoothing pass
     TbMaps tb_maps[kMaxLevels];
     int tb_zchunk[kMaxLevels] = {};
@@ -114,11 +115,16 @@ cudaError_t host_malloc(void **p, size_t bytes);
 // The red-black SOR update of one cell from its neighbour sum and right-hand
 // side (MG/MultiGrid_kernel.cu:766, omega = 1.43f, 1 - omega formed in
 // float), one expression for every smoother kernel so that they round alike.
+// The corrected cycle's (mg.cu) has its own factor, and inv = 1 / diagonal.
+constexpr float kCorrOmega = 1.25f;
 constexpr float kOmegaF = 1.43f;
 constexpr float kOneMinusOmegaF = 1.0f - 1.43f;
 __device__ __forceinline__ float mg_sor_update(float x, float nb, float b) {
     const float r = nb - b;
     return kOneMinusOmegaF * x + (kOmegaF * r) * (1.0f / 6.0f);
+}
+__device__ __forceinline__ float mg_corr_update(float x, float nb, float b, float inv) {
+    return (1.0f - kCorrOmega) * x + kCorrOmega * ((nb - b) * inv);
 }
 #endif
 
@@ -141,10 +147,8 @@ enum TailMode { kTailCycle = 0, kTailFull = 1, kTailCorrected = 2 };
 cudaError_t mg_tail_launch(const MGPlan &m, int level, TailMode mode);
 // One red-black sweep of a level of edge > 32 (mg_sweep.cu).
 cudaError_t mg_sweep_prepare();
-// The corrected cycle's ghost factor of a level (0 on the finest), and its
-// relaxation factor (mg.cu).
+// The corrected cycle's ghost factor of a level (0 on the finest; mg.cu).
 float mg_ghost_factor(int level);
-constexpr float kCorrOmega = 1.25f;
 struct SweepSpec {
     const float *x = nullptr;   // null: from zero
     const float *b = nullptr;

@@ -76,7 +76,7 @@ def test_vcycle_of_a_slice_at_an_odd_offset(pb, oracle, n):
 def test_corrected_cycles_reach_the_tolerance(pb, oracle, n, tol):
     """The solve to a tolerance: the residual of what it returns, in numpy's
     64 bits, and the number of cycles.  A cycle gains at least a factor 10
-    (0.02 on the edges measured), so 10 of them reach 1e-10 from the first's."""
+    (0.032 is the worst measured), so 10 of them reach 1e-10 from the first's."""
     import torch
     rng = np.random.default_rng(n)
     b = rng.standard_normal(n ** 3)
@@ -96,7 +96,7 @@ def test_corrected_cycles_reach_the_tolerance(pb, oracle, n, tol):
 def test_corrected_cycles_on_smooth_sources(pb, oracle, n, kind):
     """Sources whose solution lives on the coarse levels, where white noise
     (above) leaves little: 8 cycles, the first counting for two, at no more than
-    a tenth each (0.03 is the worst seen) reach 1e-8 from any of them."""
+    a tenth each (0.032 is the worst measured) reach 1e-8 from any of them."""
     import torch
     c = (np.arange(n) + 0.5) / n
     z, y, x = np.meshgrid(c, c, c, indexing="ij")
